@@ -62,7 +62,7 @@ void proton_raytrace_core(DeviceContext &ctx, const Grid &g, const Frame &f, flo
 
 // Uploads the spot/layer tables (via pinned staging) and launches the pencil beam.
 // Layer and spot tables on the device (through a pinned staging slot) and
-// the layers' cut-off radii, enqueued on s.
+// the layers' device-side entries, enqueued on s.
 ProtonTables proton_tables(DeviceContext &ctx, const Grid &g, const Frame &f, const std::vector<LayerRec> &layers,
                            const std::vector<SpotRec> &spots, const float *lut_d, const float *lut_s,
                            const float *lut_i, int lut_len, cudaStream_t s) {
@@ -76,18 +76,22 @@ ProtonTables proton_tables(DeviceContext &ctx, const Grid &g, const Frame &f, co
     char *pin = static_cast<char *>(ctx.pin_ring[slot].ensure(lb_al + sb));
     std::memcpy(pin, layers.data(), lb);
     std::memcpy(pin + lb_al, spots.data(), sb);
-    char *dev = static_cast<char *>(ctx.tables.ensure(lb_al + sb));
+    const size_t rows_off = lb_al + ((sb + 255) & ~(size_t)255);
+    const size_t axes_off = rows_off + layers.size() * (lut_len + 1) * sizeof(float4);
+    char *dev = static_cast<char *>(ctx.tables.ensure(axes_off + spots.size() * sizeof(float4)));
     DC_CUDA(cudaMemcpyAsync(dev, pin, lb_al + sb, cudaMemcpyHostToDevice, s));
     DC_CUDA(cudaEventRecord(ctx.pin_ev[slot], s));
-    launch_layer_rcut(g, f, reinterpret_cast<LayerRec *>(dev), (int)layers.size(), lut_d, lut_s, lut_len, s);
     ProtonTables t;
     t.layers = reinterpret_cast<const LayerRec *>(dev);
     t.spots = reinterpret_cast<const SpotRec *>(dev + lb_al);
     t.lut_depths = lut_d;
     t.lut_sigmas = lut_s;
     t.lut_idds = lut_i;
+    t.rows = reinterpret_cast<const float4 *>(dev + rows_off);
+    t.axes = reinterpret_cast<const float4 *>(dev + axes_off);
     t.n_layers = (int)layers.size();
     t.lut_len = lut_len;
+    launch_layer_tables(g, f, t, s);
     return t;
 }
 
@@ -131,7 +135,7 @@ int dc_debug_bounds(int gpu_id, unsigned long long *violation, int *enabled) {
         unsigned long long v = 0;
         for (unsigned long long w : {take_bounds_wet(), take_bounds_photon(), take_bounds_proton(),
                                      take_bounds_basis(), take_bounds_noalloc(), take_bounds_xray(),
-                                     take_bounds_fluence(), take_bounds_sweep()})
+                                     take_bounds_fluence(), take_bounds_sweep(), take_bounds_pencil()})
             if (v == 0) v = w;
         *violation = v;
     });

@@ -5,7 +5,7 @@
 // A batch holds any number of plans (each with its own CT grid, RLSP volume
 // and dose volume) and beams (each with its own geometry, spot list and WET
 // volume) resident on one device.  Its dose call is a single persistent
-// kernel whose CTAs take (plan, tile) work items from a device queue sorted
+// kernel whose warps take (plan, tile) work items from a device queue sorted
 // by plan cost, so plans with uneven spot and beam counts share the GPU
 // without a tail; each item sums its plan's beams layer by layer (energy
 // order) in registers and writes each voxel once.  The WET call runs the ray
@@ -43,7 +43,7 @@ struct HostBeam {
     float *wet;  // device
     std::vector<LayerRec> layers;
     std::vector<SpotRec> spots;
-    size_t layer_off = 0, spot_off = 0;  // byte offsets in the table buffer
+    size_t layer_off = 0, spot_off = 0, rows_off = 0, axes_off = 0;  // byte offsets in the table buffer
     int spot_base = 0;                   // offset in the batch's spot-weight vector
 };
 
@@ -62,10 +62,10 @@ struct dc_proton_batch {
     size_t lut_stride = 0;
     DeviceBuffer tables;    // per-beam LayerRec[] and SpotRec[]
     DeviceBuffer mu;        // float[n_spots_total]: the spot weights the dose uses
-    DeviceBuffer d_plans;   // PbBatchPlan[]
+    DeviceBuffer d_plans;   // PbBatchPlan[], most expensive first
     DeviceBuffer d_beams;   // PbBatchBeam[]
-    DeviceBuffer d_items[8];
-    int n_items[8] = {0};
+    DeviceBuffer first_tile;  // int64[n_plans + 1], in the order of d_plans
+    long long n_items = 0;
     DeviceBuffer queue;     // unsigned queue head
     DeviceBuffer wet_raw;   // unsmoothed WET scratch (largest plan)
     std::vector<std::unique_ptr<VolumeArray>> arrays;  // per-plan RLSP texture
@@ -83,7 +83,7 @@ struct dc_proton_batch {
         mu.release();
         d_plans.release();
         d_beams.release();
-        for (auto &b : d_items) b.release();
+        first_tile.release();
         queue.release();
         wet_raw.release();
         for (auto &a : arrays) a->release();
@@ -208,6 +208,10 @@ int dc_proton_batch_commit(dc_proton_batch *b) {
             off = align256(off + hb.layers.size() * sizeof(LayerRec));
             hb.spot_off = off;
             off = align256(off + hb.spots.size() * sizeof(SpotRec));
+            hb.rows_off = off;
+            off = align256(off + hb.layers.size() * (b->lut_len + 1) * sizeof(float4));
+            hb.axes_off = off;
+            off = align256(off + hb.spots.size() * sizeof(float4));
             hb.spot_base = spot_base;
             spot_base += (int)hb.spots.size();
         }
@@ -232,8 +236,6 @@ int dc_proton_batch_commit(dc_proton_batch *b) {
         for (auto &p : b->plans) {
             for (size_t q = 0; q < p.beams.size(); ++q, ++bi) {
                 HostBeam &hb = b->beams[bi];
-                launch_layer_rcut(p.g, hb.f, reinterpret_cast<LayerRec *>(tab + hb.layer_off), (int)hb.layers.size(),
-                                  lut_d, lut_s, b->lut_len, nullptr);
                 PbBatchBeam B;
                 B.f = hb.f;
                 B.t.layers = reinterpret_cast<const LayerRec *>(tab + hb.layer_off);
@@ -241,8 +243,11 @@ int dc_proton_batch_commit(dc_proton_batch *b) {
                 B.t.lut_depths = lut_d;
                 B.t.lut_sigmas = lut_s;
                 B.t.lut_idds = lut_i;
+                B.t.rows = reinterpret_cast<const float4 *>(tab + hb.rows_off);
+                B.t.axes = reinterpret_cast<const float4 *>(tab + hb.axes_off);
                 B.t.n_layers = (int)hb.layers.size();
                 B.t.lut_len = b->lut_len;
+                launch_layer_tables(p.g, hb.f, B.t, nullptr);
                 B.wet = hb.wet;
                 B.mu = mu + hb.spot_base;
                 hbeams.push_back(B);
@@ -261,29 +266,26 @@ int dc_proton_batch_commit(dc_proton_batch *b) {
             hplans.push_back(P);
             max_vox = std::max(max_vox, p.g.n());
         }
-        void *dp = b->d_plans.ensure(hplans.size() * sizeof(PbBatchPlan));
-        DC_CUDA(cudaMemcpy(dp, hplans.data(), hplans.size() * sizeof(PbBatchPlan), cudaMemcpyHostToDevice));
         void *db = b->d_beams.ensure(hbeams.size() * sizeof(PbBatchBeam));
         DC_CUDA(cudaMemcpy(db, hbeams.data(), hbeams.size() * sizeof(PbBatchBeam), cudaMemcpyHostToDevice));
         b->hbeams = hbeams;
-        // work queues, one per tile shape: plans by decreasing cost, tiles in order
+        // work queue: plans by decreasing cost, tiles in order
         std::vector<int> plan_order(b->plans.size());
         std::iota(plan_order.begin(), plan_order.end(), 0);
         std::stable_sort(plan_order.begin(), plan_order.end(),
                          [&](int x, int y) { return b->plans[x].cost > b->plans[y].cost; });
-        const int nv = pencil_beam_batch_variants();
-        for (int v = 0; v < nv && v < 8; ++v) {
-            std::vector<int2> items;
-            for (int pi : plan_order) {
-                const long long tiles = pencil_beam_batch_tiles(v, b->plans[pi].g);
-                need(tiles < 0x7fffffffLL, "plan too large for the batch work queue.");
-                for (long long t = 0; t < tiles; ++t) items.push_back(make_int2(pi, (int)t));
-            }
-            need(items.size() < 0x7fffffffULL, "batch too large for the work queue.");
-            void *ip = b->d_items[v].ensure(items.size() * sizeof(int2));
-            DC_CUDA(cudaMemcpy(ip, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice));
-            b->n_items[v] = (int)items.size();
+        std::vector<PbBatchPlan> queued;
+        std::vector<long long> first(1, 0);
+        for (int pi : plan_order) {
+            queued.push_back(hplans[pi]);
+            first.push_back(first.back() + pencil_beam_batch_tiles(b->plans[pi].g));
         }
+        need(first.back() < 0x7fffffffLL, "batch too large for the work queue.");
+        b->n_items = first.back();
+        void *dp = b->d_plans.ensure(queued.size() * sizeof(PbBatchPlan));
+        DC_CUDA(cudaMemcpy(dp, queued.data(), queued.size() * sizeof(PbBatchPlan), cudaMemcpyHostToDevice));
+        void *fp = b->first_tile.ensure(first.size() * sizeof(long long));
+        DC_CUDA(cudaMemcpy(fp, first.data(), first.size() * sizeof(long long), cudaMemcpyHostToDevice));
         b->queue.ensure(sizeof(unsigned));
         b->wet_raw.ensure((size_t)max_vox * sizeof(float));
         for (auto &p : b->plans) {
@@ -356,8 +358,8 @@ int dc_proton_batch_dose(dc_proton_batch *b, const float *mu_dev, int variant, v
             DC_CUDA(cudaMemcpyAsync(b->mu.ptr, mu_dev, (size_t)b->n_spots_total * sizeof(float),
                                     cudaMemcpyDeviceToDevice, s));
         launch_pencil_beam_batch(ctx, variant, b->d_plans.as<const PbBatchPlan>(), b->d_beams.as<const PbBatchBeam>(),
-                                 b->d_items[variant].as<const int2>(), b->n_items[variant], b->queue.as<unsigned>(),
-                                 b->lut_len, s);
+                                 b->first_tile.as<const long long>(), (int)b->plans.size(), b->n_items,
+                                 b->queue.as<unsigned>(), s);
         ctx.end_call(s);
     });
 }

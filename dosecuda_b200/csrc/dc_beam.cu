@@ -35,9 +35,9 @@ struct dc_proton_beam {
     Frame f{};
     int n_spots = 0, n_layers = 0, n_energies = 0, lut_len = 0;
     long long n_vox = 0;
-    DeviceBuffer tables;  // LayerRec[n_layers] | SpotRec[n_spots]
+    DeviceBuffer tables;  // LayerRec[n_layers] | SpotRec[n_spots] | rows float4[n_layers][lut_len + 1] | axes float4[n_spots]
     DeviceBuffer luts;    // depths | sigmas | idds
-    size_t spot_off = 0, lut_stride = 0;
+    size_t spot_off = 0, rows_off = 0, axes_off = 0, lut_stride = 0;
     DeviceBuffer spot_max;  // unsigned[n_spots]
     DeviceBuffer thr;       // float[n_spots]
     DeviceBuffer counts;    // int[n_vox]
@@ -59,6 +59,8 @@ struct dc_proton_beam {
         t.lut_depths = luts.as<const float>();
         t.lut_sigmas = reinterpret_cast<const float *>(static_cast<const char *>(luts.ptr) + lut_stride);
         t.lut_idds = reinterpret_cast<const float *>(static_cast<const char *>(luts.ptr) + 2 * lut_stride);
+        t.rows = reinterpret_cast<const float4 *>(static_cast<const char *>(tables.ptr) + rows_off);
+        t.axes = reinterpret_cast<const float4 *>(static_cast<const char *>(tables.ptr) + axes_off);
         t.n_layers = n_layers;
         t.lut_len = lut_len;
         return t;
@@ -220,7 +222,9 @@ int dc_proton_beam_create(int gpu_id, int nz, int ny, int nx, const float spacin
         b->n_vox = (long long)nz * ny * nx;
         const size_t lb = layers.size() * sizeof(LayerRec);
         b->spot_off = (lb + 255) & ~(size_t)255;
-        void *tp = b->tables.ensure(b->spot_off + recs.size() * sizeof(SpotRec));
+        b->rows_off = (b->spot_off + recs.size() * sizeof(SpotRec) + 255) & ~(size_t)255;
+        b->axes_off = b->rows_off + layers.size() * (lut_len + 1) * sizeof(float4);
+        void *tp = b->tables.ensure(b->axes_off + recs.size() * sizeof(float4));
         DC_CUDA(cudaMemcpy(tp, layers.data(), lb, cudaMemcpyHostToDevice));
         DC_CUDA(cudaMemcpy(static_cast<char *>(tp) + b->spot_off, recs.data(), recs.size() * sizeof(SpotRec),
                            cudaMemcpyHostToDevice));
@@ -230,8 +234,7 @@ int dc_proton_beam_create(int gpu_id, int nz, int ny, int nx, const float spacin
         DC_CUDA(cudaMemcpy(lp, lut_depths, lbytes, cudaMemcpyHostToDevice));
         DC_CUDA(cudaMemcpy(lp + b->lut_stride, lut_sigmas, lbytes, cudaMemcpyHostToDevice));
         DC_CUDA(cudaMemcpy(lp + 2 * b->lut_stride, lut_idds, lbytes, cudaMemcpyHostToDevice));
-        launch_layer_rcut(b->g, b->f, static_cast<LayerRec *>(tp), b->n_layers, reinterpret_cast<const float *>(lp),
-                          reinterpret_cast<const float *>(lp + b->lut_stride), lut_len, nullptr);
+        launch_layer_tables(b->g, b->f, b->view(), nullptr);
         DC_CUDA(cudaDeviceSynchronize());
         *out = b.release();
     });
@@ -279,7 +282,7 @@ int dc_proton_beam_adjoint(dc_proton_beam *b, const float *wet_dev, const float 
         PbExtra x;
         x.grad_dose = grad_dose_dev;
         x.grad_mu = grad_mu_dev;
-        launch_pencil_beam_mode(ctx, kPbAdjoint, b->g, b->f, b->view(), wet_dev, x, s);
+        launch_pencil_beam_adjoint(ctx, b->g, b->f, b->view(), wet_dev, x, s);
         ctx.end_call(s);
     });
 }

@@ -45,21 +45,29 @@ void launch_xray_depth(DeviceContext &ctx, const Grid &g, const Frame &f, cudaTe
                        int *list, unsigned *n_list, DeviceBuffer &lattice, unsigned *stats, float wet_exact,
                        cudaStream_t s);
 
-// ---- proton pencil beam (dc_proton.cu) -----------------------------------
+// ---- proton pencil beam (tables and influence: dc_proton.cu; dose and
+// adjoint: dc_pencil.cu) -----------------------------------
 // One energy layer: a run of spots with the same energy id
 // (reference Layer, IMPTClasses.cuh:17-26; importLayers IMPTClasses.cu:37-67).
-struct LayerRec {
+// The fields lie in 16-byte groups, which dc_pencil.cu loads as such.
+struct __align__(16) LayerRec {
     int spot_start;
     int n_spots;
     int energy_id;
     float r80;
     float A, B, C;  // sigma_air quadratic coefficients (divergence_params[2..4])
-    float rcut;     // lateral cut-off radius (mm): 6 x the widest halo sigma of the layer
+    float rcut;     // lateral cut-off radius (mm): 6 x the widest halo sigma of the layer (device)
+    float x0, x1, y0, y1;    // range of the layer's spot positions
+    float inv_vx, inv_vy;    // 1 / VSADX, 1 / VSADY
+    float it2_min;           // smallest SpotRec::inv_t2 of the layer
+    // device: first depth of the layer's LUT row, 1 / step and step (0 unless
+    // the depths are evenly spaced)
+    float lut_d0, lut_inv, lut_step;
+    // device: coefficients of the nuclear halo's sigma (log and pole terms)
+    // and weight (log argument, quotient, linear term) at this R80
+    float hs_log, hs_pole, hw_arg, hw_num, hw_den, hw_lin;
 };
 
-// Fills LayerRec::rcut on the device from the LUT rows (layer_rcut_kernel).
-void launch_layer_rcut(const Grid &g, const Frame &f, LayerRec *layers, int n_layers, const float *lut_depths,
-                       const float *lut_sigmas, int lut_len, cudaStream_t s);
 
 // Spot record with the divergent-axis constants precomputed on the host:
 // t = (x/VSADX, y/VSADY, -1), inv_t2 = 1/|t|^2 (IMPTClasses.cu:123-133).
@@ -77,9 +85,19 @@ struct ProtonTables {
     const float *lut_depths;  // [n_energies][lut_len]
     const float *lut_sigmas;
     const float *lut_idds;
+    const float4 *rows;       // [n_layers][lut_len + 1] and
+    const float4 *axes;       // [n_spots], see launch_layer_tables
     int n_layers;
     int lut_len;
 };
+
+// Device part of the layer and spot tables (layer_tables_kernel), written
+// through t's pointers: LayerRec's device fields; rows[layer][i], i = 0 ..
+// lut_len, = sigma and idd at depth i - 1 and their steps to depth i (no step
+// at the ends), so that a voxel's lookup reads one 16-byte record; and per spot
+// axes = (p, q, k1, r): the vectors (p, q, k1) and (0, r, r ty) are orthonormal
+// and normal to the spot's axis t = (tx, ty, -1).
+void launch_layer_tables(const Grid &g, const Frame &f, const ProtonTables &t, cudaStream_t s);
 
 // Per-mode inputs/outputs of the pencil-beam kernel family (all device
 // pointers; spot-indexed arrays are in the caller's spot order).
@@ -112,6 +130,7 @@ enum PbMode { kPbDose = 0, kPbAdjoint = 1, kPbSpotMax = 2, kPbCount = 3, kPbFill
 unsigned long long take_bounds_wet();
 unsigned long long take_bounds_photon();
 unsigned long long take_bounds_proton();
+unsigned long long take_bounds_pencil();
 unsigned long long take_bounds_basis();
 unsigned long long take_bounds_noalloc();
 unsigned long long take_bounds_xray();
@@ -127,7 +146,7 @@ void build_proton_tables(const float *spots, int n_spots, const float *dvp, int 
 void launch_pencil_beam(DeviceContext &ctx, const Grid &g, const Frame &f, const ProtonTables &t,
                         const float *wet_s, float *dose, cudaStream_t s, const float *mu_dev = nullptr,
                         int tile_z0 = 0, int tile_z1 = -1);
-// Voxels along z per tile of the single-beam pencil-beam kernel: tiles
+// Voxels along z per tile of the one-beam pencil-beam kernel: tiles
 // [z0, z1) cover planes [z0 * depth, z1 * depth).
 int pencil_beam_tile_depth();
 // Dose (x.list_out) or adjoint (x.grad_dose compact, x.grad_mu) of the voxels
@@ -135,7 +154,11 @@ int pencil_beam_tile_depth();
 void launch_pencil_beam_list(DeviceContext &ctx, int mode, const Grid &g, const Frame &f, const ProtonTables &t,
                              const float *wet_s, const PbExtra &x, cudaStream_t s);
 
-// The other members of the family (see PbMode); `name` labels the profiler entry.
+// x.grad_mu[s] += sum over the volume of x.grad_dose(v) K_s(v).
+void launch_pencil_beam_adjoint(DeviceContext &ctx, const Grid &g, const Frame &f, const ProtonTables &t,
+                                const float *wet_s, const PbExtra &x, cudaStream_t s);
+
+// The influence passes: kPbSpotMax, kPbCount, kPbFill.
 void launch_pencil_beam_mode(DeviceContext &ctx, int mode, const Grid &g, const Frame &f, const ProtonTables &t,
                              const float *wet_s, const PbExtra &x, cudaStream_t s);
 
@@ -164,13 +187,14 @@ struct PbBatchPlan {
     int beam0, n_beams;
 };
 
-// Work items are (plan, tile) pairs; tile = bz * tiles_x * tiles_y + by * tiles_x + bx
-// for the variant's tile shape.  `next` is the device queue head (reset here).
+// Work items are (plan, tile) pairs in the order of `plans`: plan q's items
+// are first_tile[q] .. first_tile[q + 1] - 1 (device array of n_plans + 1).
+// `next` is the device queue head (reset here).
 int pencil_beam_batch_variants();
-void pencil_beam_batch_tile(int variant, int *threads_y, int *voxels_per_thread);
-long long pencil_beam_batch_tiles(int variant, const Grid &g);  // tiles of grid g
+long long pencil_beam_batch_tiles(const Grid &g);  // tiles of grid g
 void launch_pencil_beam_batch(DeviceContext &ctx, int variant, const PbBatchPlan *plans, const PbBatchBeam *beams,
-                              const int2 *items, int n_items, unsigned *next, int lut_len, cudaStream_t s);
+                              const long long *first_tile, int n_plans, long long n_items, unsigned *next,
+                              cudaStream_t s);
 
 // Piecewise-linear HU table (strictly increasing HU), kernel parameter.
 constexpr int kMaxHuPoints = 64;

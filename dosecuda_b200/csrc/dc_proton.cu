@@ -1,4 +1,6 @@
-// dc_proton.cu — double-Gaussian proton pencil-beam dose.
+// dc_proton.cu — double-Gaussian proton pencil beam: layer and spot tables,
+// and the dose-influence passes (spot maxima, count, fill).  The dose and its
+// adjoint are in dc_pencil.cu.
 //
 // Restates pencilBeamKernel (IMPTClasses.cu:204-271) and its helpers
 // (interpolateProtonLUT :69-92, sigmaAir :94-102, nuclearHalo :104-121,
@@ -14,18 +16,12 @@
 // with r^2 the squared distance from the voxel (BEV coordinates) to the
 // spot's divergent axis.
 //
-// B200 mapping (instead of one thread per (voxel, layer) with a global
-// atomicAdd per pair of the reference): a CTA owns a 16x8x4 tile of voxels,
-// two voxels per thread, and walks all energy layers.  Per layer
-// the CTA stages the layer's LUT rows and spot records in shared memory
-// (broadcast reads in the spot loop); each thread keeps its voxels' dose in
-// registers across layers and writes each voxel once — no atomics, so the
-// result is deterministic.  The spot loop is two exponentials per
-// (voxel, spot) pair on the special-function unit (ex2.approx with the
-// log2(e) factor folded into the per-voxel Gaussian scales) plus ~12 FP32
-// operations.  The FP32 part runs on the paired-lane f32x2 instructions of
-// sm_100 (a thread's two voxels share one issue; same IEEE operations, same
-// bits), which leaves the kernel bound by the SFU rate and instruction issue.
+// The influence passes keep their entries' values and their threshold test in
+// one kernel instantiation (see below): a CTA owns a 16x8x4 tile of voxels,
+// two voxels per thread, walks all energy layers, and per layer stages the
+// LUT rows and spot records in shared memory (broadcast reads in the spot
+// loop).  The FP32 part runs on the paired-lane f32x2 instructions of sm_100
+// (a thread's two voxels share one issue; same IEEE operations, same bits).
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -129,7 +125,21 @@ void build_proton_tables(const float *spots, int n_spots, const float *dvp, int 
         L.A = row[2];
         L.B = row[3];
         L.C = row[4];
-        L.rcut = INFINITY;  // set on the device by layer_rcut_kernel
+        L.rcut = INFINITY;  // set on the device by layer_tables_kernel
+        L.x0 = L.y0 = INFINITY;
+        L.x1 = L.y1 = -INFINITY;
+        L.it2_min = 1.0f;
+        for (int q = s; q < t; ++q) {
+            L.x0 = std::min(L.x0, spot_recs[q].x);
+            L.x1 = std::max(L.x1, spot_recs[q].x);
+            L.y0 = std::min(L.y0, spot_recs[q].y);
+            L.y1 = std::max(L.y1, spot_recs[q].y);
+            L.it2_min = std::min(L.it2_min, spot_recs[q].inv_t2);
+        }
+        L.inv_vx = 1.0f / vsadx;
+        L.inv_vy = 1.0f / vsady;
+        L.lut_d0 = L.lut_inv = L.lut_step = 0.0f;
+        L.hs_log = L.hs_pole = L.hw_arg = L.hw_num = L.hw_den = L.hw_lin = 0.0f;
         layers.push_back(L);
         s = t;
     }
@@ -224,15 +234,32 @@ __device__ __forceinline__ float2 exp2_pair(float2 x) { return make_float2(fast_
 //  * |sigma_air| by the quadratic's extremes over the range of
 //    d = |voxel - source| - w + 0.7 R80 for voxels of the volume;
 //  * sigma_h by sampling the halo formula over [0.1, R80 - 0.1] mm.
-// One warp per layer: the lanes share the LUT scan and the halo-sigma
-// samples, and the maxima are combined with shuffles.
-__global__ void __launch_bounds__(32) layer_rcut_kernel(Grid g, Frame f, LayerRec *layers, int n_layers,
-                                                        const float *lut_depths, const float *lut_sigmas,
-                                                        int lut_len) {
+// One block per layer: the first warp's lanes share the LUT scan and the
+// halo-sigma samples and combine the maxima with shuffles; the other warps
+// write the layer's LUT rows and spot axes for dc_pencil.cu.
+__global__ void __launch_bounds__(128) layer_tables_kernel(Grid g, Frame f, ProtonTables t) {
     const int l = blockIdx.x;
     const int lane = threadIdx.x;
-    if (l >= n_layers) return;
-    LayerRec &L = layers[l];
+    if (l >= t.n_layers) return;
+    LayerRec &L = const_cast<LayerRec *>(t.layers)[l];
+    const int lut_len = t.lut_len;
+    if (lane >= 32) {
+        const size_t at = (size_t)L.energy_id * lut_len;
+        float4 *rows = const_cast<float4 *>(t.rows) + (size_t)l * (lut_len + 1);
+        for (int q = lane - 32; q <= lut_len; q += (int)blockDim.x - 32) {
+            const size_t lo = at + max(q - 1, 0), hi = at + min(q, lut_len - 1);
+            const float s0 = t.lut_sigmas[lo], i0 = t.lut_idds[lo];
+            rows[q] = make_float4(s0, i0, t.lut_sigmas[hi] - s0, t.lut_idds[hi] - i0);
+        }
+        float4 *axes = const_cast<float4 *>(t.axes) + L.spot_start;
+        for (int q = lane - 32; q < L.n_spots; q += (int)blockDim.x - 32) {
+            const SpotRec &s = t.spots[L.spot_start + q];
+            const float a = fmaf(s.ty, s.ty, 1.0f) * s.inv_t2;
+            const float p = sqrtf(a), b = -(s.tx * s.ty * s.inv_t2) / p;
+            axes[q] = make_float4(p, b, fmaf(p, s.tx, b * s.ty), sqrtf(s.inv_t2 / a));
+        }
+        return;
+    }
     // source distance range over the volume's bounding box (image frame, relative to iso)
     const float lo[3] = {-f.isox - 0.5f * g.sx, -f.isoy - 0.5f * g.sy, -f.isoz - 0.5f * g.sz};
     const float hi[3] = {(g.nx - 0.5f) * g.sx - f.isox, (g.ny - 0.5f) * g.sy - f.isoy, (g.nz - 0.5f) * g.sz - f.isoz};
@@ -245,8 +272,12 @@ __global__ void __launch_bounds__(32) layer_rcut_kernel(Grid g, Frame f, LayerRe
     }
     const float r80 = L.r80;
     const float wmax = 1.1f * r80;
-    const float *D = lut_depths + (size_t)L.energy_id * lut_len;
-    const float *S = lut_sigmas + (size_t)L.energy_id * lut_len;
+    const float *D = t.lut_depths + (size_t)L.energy_id * lut_len;
+    const float *S = t.lut_sigmas + (size_t)L.energy_id * lut_len;
+    const float step = lut_len > 1 ? (D[lut_len - 1] - D[0]) / (float)(lut_len - 1) : 0.0f;
+    bool even = step > 0.0f;
+    for (int q = lane; q < lut_len; q += 32) even = even && D[q] == fmaf((float)q, step, D[0]);
+    even = __all_sync(0xffffffffu, even);
     // |sigma| over the rows up to the first one deeper than wmax (that row
     // included: it brackets wmax from above)
     int q_end = lut_len;
@@ -287,22 +318,26 @@ __global__ void __launch_bounds__(32) layer_rcut_kernel(Grid g, Frame f, LayerRe
     }
     const float sht = hypotf(sa + smcs, sh * 1.02f + 0.2f) * 1.01f + 0.5f;
     L.rcut = (sht == sht) ? 6.0f * sht : INFINITY;
+    L.lut_d0 = D[0];
+    L.lut_inv = even ? 1.0f / step : 0.0f;
+    L.lut_step = even ? step : 0.0f;
+    L.hs_log = 0.0014f * r80 * CUDART_LN2_F;
+    L.hs_pole = 0.22f * r80;
+    L.hw_arg = 1.0f / (11.2f - 0.023f * r80);
+    L.hw_num = 0.35f * ((0.0017f * sqr(r80)) - r80);
+    L.hw_den = sqr(r80 + 3.0f);
+    L.hw_lin = 1.61e-9f * sqr(r80 + 3.0f);
 }
 
-void launch_layer_rcut(const Grid &g, const Frame &f, LayerRec *layers, int n_layers, const float *lut_depths,
-                       const float *lut_sigmas, int lut_len, cudaStream_t s) {
-    if (n_layers <= 0) return;
-    layer_rcut_kernel<<<n_layers, 32, 0, s>>>(g, f, layers, n_layers, lut_depths, lut_sigmas, lut_len);
-    check_launch("layer_rcut_kernel");
+void launch_layer_tables(const Grid &g, const Frame &f, const ProtonTables &t, cudaStream_t s) {
+    if (t.n_layers <= 0) return;
+    layer_tables_kernel<<<t.n_layers, 128, 0, s>>>(g, f, t);
+    check_launch("layer_tables_kernel");
 }
 
-// The pencil-beam kernel family.  Every member walks the same tiles, layers
-// and spots and evaluates the same per-pair influence
-//   K_s(v) = pf exp2(ps2 r^2) + hf exp2(hs2 r^2)   (dose per MU),
-// so the dose, its adjoint and the influence matrix agree to rounding.
-//   kPbDose     dose(v)       = sum_s mu_s K_s(v)          (one write per voxel)
-//   kPbAdjoint  grad_mu[s]   += sum_v g(v) K_s(v)          (warp reduction per spot,
-//                                                           one FP64 atomic per CTA and spot)
+// The influence passes.  Each walks the same tiles, layers and spots and
+// evaluates the same per-pair influence
+//   K_s(v) = pf exp2(ps2 r^2) + hf exp2(hs2 r^2)   (dose per MU).
 //   kPbSpotMax  spot_max[s]   = max_v K_s(v)
 //   kPbCount    counts[v]     = #{s : K_s(v) >= thr[s]}
 //   kPbFill     CSR row v     = (s, K_s(v)) for K_s(v) >= thr[s], in spot-table order
@@ -312,17 +347,13 @@ void launch_layer_rcut(const Grid &g, const Frame &f, LayerRec *layers, int n_la
 //               code; separately compiled, the per-voxel parameters' plain
 //               FP32 expressions may be contracted differently and a pair
 //               at its threshold may flip between the passes)
-//   list mode   the CTA's voxels are x.list[bx*(threads*VY) + v*threads + tid]
-//               instead of an image tile (dose / adjoint of listed voxels)
-template <int kMode, int TY, int VY, bool kList = false>
+template <int kMode, int TY, int VY>
 __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const ProtonTables &t,
-                                        const float *__restrict__ wet_s, int bx, int by, int bz, float (&acc)[VY],
-                                        const PbExtra &x) {
+                                        const float *__restrict__ wet_s, int bx, int by, int bz, const PbExtra &x) {
     extern __shared__ float4 smem4[];
     float4 *s_spot_a = smem4;                    // x, y, mu, orig (int bits)
     float4 *s_spot_b = smem4 + kPbSpotChunk;     // tx, ty, inv_t2, threshold
-    float *s_acc = reinterpret_cast<float *>(smem4 + 2 * kPbSpotChunk);  // adjoint partial sums
-    float *s_lut = s_acc + kPbSpotChunk;
+    float *s_lut = reinterpret_cast<float *>(smem4 + 2 * kPbSpotChunk);
     float *s_depth = s_lut;
     float *s_sigma = s_lut + t.lut_len;
     float *s_idd = s_lut + 2 * t.lut_len;
@@ -333,36 +364,18 @@ __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const Pro
     const int tid = threadIdx.y * kPbThreadsX + threadIdx.x;
     const int lane = threadIdx.x;
     const int nthreads = kThreads;
-    __syncthreads();  // shared memory of a previous tile (persistent caller) no longer in use
 
     float hx[VY], hy[VY], hz[VY], wet_mm[VY], dsrc[VY];
-    float gv[VY];
     long long vidx[VY];
     long long fill_off[VY], fill_end[VY];
     int cnt[VY];
     bool inside[VY];
 #pragma unroll
     for (int v = 0; v < VY; ++v) {
-        int ic, jc, kc;
-        if constexpr (kList) {
-            const int e = bx * (kThreads * VY) + v * kThreads + tid;
-            const long long plane = (long long)g.nx * g.ny;
-            long long vi = x.list[min(e, x.n_list - 1)];
-            const bool valid = vi >= 0 && vi < plane * g.nz;  // out-of-grid entries give 0
-            inside[v] = e < x.n_list && valid;
-            vidx[v] = valid ? vi : 0;
-            kc = (int)(vidx[v] / plane);
-            const long long rem = vidx[v] - (long long)kc * plane;
-            jc = (int)(rem / g.nx);
-            ic = (int)(rem - (long long)jc * g.nx);
-        } else {
-            const int3 q = pb_tile_voxel<TY, VY>(bx, by, bz, v);
-            inside[v] = q.x < g.nx && q.y < g.ny && q.z < g.nz;
-            ic = min(q.x, g.nx - 1);
-            jc = min(q.y, g.ny - 1);
-            kc = min(q.z, g.nz - 1);
-            vidx[v] = (long long)ic + (long long)g.nx * (jc + (long long)g.ny * kc);
-        }
+        const int3 q = pb_tile_voxel<TY, VY>(bx, by, bz, v);
+        inside[v] = q.x < g.nx && q.y < g.ny && q.z < g.nz;
+        const int ic = min(q.x, g.nx - 1), jc = min(q.y, g.ny - 1), kc = min(q.z, g.nz - 1);
+        vidx[v] = (long long)ic + (long long)g.nx * (jc + (long long)g.ny * kc);
         cnt[v] = 0;
         const float3 p = voxel_xyz(g, f, ic, jc, kc);
         const float3 h = image_to_head<false>(f, p);
@@ -371,13 +384,6 @@ __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const Pro
         hz[v] = h.z;
         dsrc[v] = distance_to_source(f, p);
         wet_mm[v] = (DC_IN_BOUNDS(vidx[v], g.n(), 21) ? __ldg(wet_s + vidx[v]) : 0.0f) * 10.0f;
-        gv[v] = 0.0f;
-        if (kMode == kPbAdjoint) {
-            if constexpr (kList)
-                gv[v] = inside[v] ? __ldg(x.grad_dose + bx * (kThreads * VY) + v * kThreads + tid) : 0.0f;
-            else
-                gv[v] = inside[v] ? __ldg(x.grad_dose + vidx[v]) : 0.0f;
-        }
         fill_off[v] = fill_end[v] = 0;
         if (kMode == kPbCount && x.row_ptr != nullptr && inside[v]) {
             fill_off[v] = x.row_ptr[vidx[v]];
@@ -463,10 +469,6 @@ __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const Pro
 #pragma unroll
         for (int v = 0; v < VY; ++v) {
             act[v] = inside[v] && pb_voxel_layer(L, s_depth, s_sigma, s_idd, t.lut_len, wet_mm[v], dsrc[v], pv[v]);
-            // adjoint: a voxel with zero gradient adds exactly zero to every
-            // spot's sum, so it counts as inactive (an objective's gradient
-            // vanishes outside its voxel sets)
-            if (kMode == kPbAdjoint) act[v] = act[v] && gv[v] != 0.0f;
             if (!act[v]) {
                 pv[v].pf = pv[v].hf = 0.f;
                 pv[v].ps2 = pv[v].hs2 = 0.f;
@@ -545,71 +547,16 @@ __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const Pro
                 if (!keep[u]) continue;
                 float4 a = a2[u], b = b2[u];
                 const int orig = __float_as_int(a.w);
-                if (x.mu) a.z = __ldg(x.mu + orig);
                 if (kMode == kPbCount) b.w = __ldg(x.thr + orig);
                 s_spot_a[pos] = a;
                 s_spot_b[pos] = b;
-                if (kMode == kPbAdjoint) s_acc[pos] = 0.0f;
                 ++pos;
             }
             __syncthreads();
             if (cn == 0) continue;
-            if constexpr (kMode == kPbDose && VY % 2 == 0) {
-                if (!any) continue;
-                // voxels (2p, 2p+1) of the thread share the paired lanes of p
-                constexpr int VP = VY / 2;
-                float2 hxp[VP], hyp[VP], hzp[VP], ps2p[VP], hs2p[VP], accp[VP], acch[VP];
-#pragma unroll
-                for (int p = 0; p < VP; ++p) {
-                    hxp[p] = make_float2(hx[2 * p], hx[2 * p + 1]);
-                    hyp[p] = make_float2(hy[2 * p], hy[2 * p + 1]);
-                    hzp[p] = make_float2(hz[2 * p], hz[2 * p + 1]);
-                    ps2p[p] = make_float2(pv[2 * p].ps2, pv[2 * p + 1].ps2);
-                    hs2p[p] = make_float2(pv[2 * p].hs2, pv[2 * p + 1].hs2);
-                    accp[p] = acch[p] = f2(0.f);
-                }
-#pragma unroll 4
-                for (int q = 0; q < cn; ++q) {
-                    const float4 a = s_spot_a[q];
-                    const float4 b = s_spot_b[q];
-                    const float2 nsx = f2(-a.x), nsy = f2(-a.y), tx = f2(b.x), ty = f2(b.y), ntx = f2(-b.x);
-                    const float2 it2 = f2(b.z), mu = f2(a.z);
-#pragma unroll
-                    for (int p = 0; p < VP; ++p) {
-                        const float2 r2 = pb_r2_pair(hxp[p], hyp[p], hzp[p], nsx, nsy, tx, ty, ntx, it2);
-                        accp[p] = __ffma2_rn(mu, exp2_pair(__fmul2_rn(ps2p[p], r2)), accp[p]);
-                        acch[p] = __ffma2_rn(mu, exp2_pair(__fmul2_rn(hs2p[p], r2)), acch[p]);
-                    }
-                }
-#pragma unroll
-                for (int p = 0; p < VP; ++p) {
-                    if (act[2 * p]) acc[2 * p] += fmaf(pv[2 * p].pf, accp[p].x, pv[2 * p].hf * acch[p].x);
-                    if (act[2 * p + 1]) acc[2 * p + 1] += fmaf(pv[2 * p + 1].pf, accp[p].y, pv[2 * p + 1].hf * acch[p].y);
-                }
-            } else if constexpr (kMode == kPbDose) {
-                if (!any) continue;
-                float accp[VY], acch[VY];
-#pragma unroll
-                for (int v = 0; v < VY; ++v) accp[v] = acch[v] = 0.f;
-#pragma unroll 4
-                for (int q = 0; q < cn; ++q) {
-                    const float4 a = s_spot_a[q];
-                    const float4 b = s_spot_b[q];
-#pragma unroll
-                    for (int v = 0; v < VY; ++v) {
-                        const float r2 = pb_r2(hx[v], hy[v], hz[v], a.x, a.y, b.x, b.y, b.z);
-                        accp[v] = fmaf(a.z, fast_exp2(pv[v].ps2 * r2), accp[v]);
-                        acch[v] = fmaf(a.z, fast_exp2(pv[v].hs2 * r2), acch[v]);
-                    }
-                }
-#pragma unroll
-                for (int v = 0; v < VY; ++v) {
-                    if (act[v]) acc[v] += fmaf(pv[v].pf, accp[v], pv[v].hf * acch[v]);
-                }
-            } else {
-                // modes that need the per-pair influence K_s(v); a warp
-                // without an active voxel contributes nothing and skips the
-                // spots as a whole (its shuffles stay warp-uniform)
+            {
+                // a warp without an active voxel contributes nothing and skips
+                // the spots as a whole (its shuffles stay warp-uniform)
                 const bool warp_any = __any_sync(0xffffffffu, any);
                 for (int q = 0; q < (warp_any ? cn : 0); ++q) {
                     const float4 a = s_spot_a[q];
@@ -639,14 +586,7 @@ __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const Pro
                                            : 0.0f;
                         }
                     }
-                    if (kMode == kPbAdjoint) {
-                        float c = 0.0f;
-#pragma unroll
-                        for (int v = 0; v < VY; ++v) c = fmaf(gv[v], kv[v], c);
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-                        if (lane == 0 && c != 0.0f) atomicAdd(&s_acc[q], c);
-                    } else if (kMode == kPbSpotMax) {
+                    if (kMode == kPbSpotMax) {
                         float m = 0.0f;
 #pragma unroll
                         for (int v = 0; v < VY; ++v) m = fmaxf(m, kv[v]);
@@ -667,13 +607,6 @@ __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const Pro
                         }
                     }
                 }
-                if (kMode == kPbAdjoint) {
-                    __syncthreads();
-                    for (int q = tid; q < cn; q += nthreads) {
-                        const float c = s_acc[q];
-                        if (c != 0.0f) atomicAdd(x.grad_mu + __float_as_int(s_spot_a[q].w), (double)c);
-                    }
-                }
             }
         }
     }
@@ -686,117 +619,19 @@ __device__ __forceinline__ void pb_tile(const Grid &g, const Frame &f, const Pro
 }
 
 
-// Minimum resident CTAs per SM the register allocation is held to: 4 CTAs
-// of 256 threads (or 8 of 128; 64 registers) for the one-shot and the
-// persistent batch kernels.  More resident warps hide the fixed-latency
-// chains of the spot loop and the per-layer barriers; measured on the adjoint
-// (0.492 -> 0.439 ms) and the batch (41.4 -> 35.2 ms for four plans at 3 CTAs
-// of 256 threads, 16.7 -> 15.2 ms at 4 with the 16 x TY x 8 tiles) with the
-// dose kernel unchanged, despite a few spilled words outside the spot loop.
-constexpr int pb_min_ctas(int ty, int per_256) { return ty >= 8 ? per_256 : 2 * per_256; }
-
-// One tile per CTA (grid = the tiles of the volume, pb_tiles).
+// One tile per CTA (grid = the tiles of the volume, pb_tiles); 4 resident CTAs
+// of 256 threads per SM (64 registers) hide the fixed-latency chains of the
+// spot loop and the per-layer barriers.
 template <int kMode, int TY, int VY>
-__global__ void __launch_bounds__(kPbThreadsX *TY, pb_min_ctas(TY, 4))
-    pb_kernel(Grid g, Frame f, ProtonTables t, const float *__restrict__ wet_s, float *__restrict__ dose, PbExtra x) {
-    float acc[VY];
-#pragma unroll
-    for (int v = 0; v < VY; ++v) acc[v] = 0.0f;
-    const int bz = (int)blockIdx.z + x.tile_z0;
-    pb_tile<kMode, TY, VY>(g, f, t, wet_s, blockIdx.x, blockIdx.y, bz, acc, x);
-    if (kMode == kPbDose) {
-#pragma unroll
-        for (int v = 0; v < VY; ++v) {
-            const int3 q = pb_tile_voxel<TY, VY>(blockIdx.x, blockIdx.y, bz, v);
-            const long long u = (long long)q.x + (long long)g.nx * (q.y + (long long)g.ny * q.z);
-            if (q.x < g.nx && q.y < g.ny && q.z < g.nz && DC_IN_BOUNDS(u, g.n(), 20)) dose[u] = acc[v];
-        }
-    }
-}
-
-// Voxel-list kernel (dose / adjoint of listed voxels; one CTA per
-// threads*VY consecutive list entries).  A sorted list keeps a CTA's voxels
-// close together, so the per-CTA spot culling stays tight.
-template <int kMode, int TY, int VY>
-__global__ void __launch_bounds__(kPbThreadsX *TY, pb_min_ctas(TY, 4))
-    pb_list_kernel(Grid g, Frame f, ProtonTables t, const float *__restrict__ wet_s, PbExtra x) {
-    float acc[VY];
-#pragma unroll
-    for (int v = 0; v < VY; ++v) acc[v] = 0.0f;
-    pb_tile<kMode, TY, VY, true>(g, f, t, wet_s, blockIdx.x, 0, 0, acc, x);
-    if (kMode == kPbDose) {
-        const int tid = threadIdx.y * kPbThreadsX + threadIdx.x;
-#pragma unroll
-        for (int v = 0; v < VY; ++v) {
-            const int e = blockIdx.x * (kPbThreadsX * TY * VY) + v * (kPbThreadsX * TY) + tid;
-            if (e < x.n_list && DC_IN_BOUNDS(e, x.n_list, 22)) x.list_out[e] = acc[v];
-        }
-    }
-}
-
-// Persistent batch kernel: CTAs take (plan, tile) work items from a device
-// queue (most expensive plans first) and sum the dose of all the plan's beams
-// for the tile in registers before one write per voxel.
-//
-// The plan and beam records are staged in shared memory and passed to pb_tile
-// by reference: their fields are then read from shared memory where used
-// instead of holding some twenty registers through the layer loop (the
-// one-beam kernels read the same fields from the kernel parameters).
-template <class T>
-__device__ __forceinline__ void pb_stage_record(T *dst, const T *__restrict__ src, int tid, int nthreads) {
-    static_assert(sizeof(T) % sizeof(int) == 0, "records are copied as words");
-    const int *s = reinterpret_cast<const int *>(src);
-    int *d = reinterpret_cast<int *>(dst);
-    for (int q = tid; q < (int)(sizeof(T) / sizeof(int)); q += nthreads) d[q] = __ldg(s + q);
-}
-
-template <int TY, int VY>
-__global__ void __launch_bounds__(kPbThreadsX *TY, pb_min_ctas(TY, 4))
-    pb_batch_kernel(const PbBatchPlan *__restrict__ plans, const PbBatchBeam *__restrict__ beams,
-                    const int2 *__restrict__ items, int n_items, unsigned *__restrict__ next) {
-    __shared__ int s_item;
-    __shared__ PbBatchPlan s_plan;
-    __shared__ PbBatchBeam s_beam;
-    const int tid = threadIdx.y * kPbThreadsX + threadIdx.x;
-    while (true) {
-        __syncthreads();  // the previous item's plan record no longer in use
-        if (tid == 0) s_item = (int)atomicAdd(next, 1u);
-        __syncthreads();
-        const int it = s_item;
-        if (it >= n_items) break;
-        const int2 w = items[it];
-        pb_stage_record(&s_plan, plans + w.x, tid, kPbThreadsX * TY);
-        __syncthreads();
-        const PbBatchPlan &P = s_plan;
-        const int3 nt = pb_tiles<TY, VY>(P.g);
-        const int bz = w.y / (nt.x * nt.y);
-        const int rem = w.y - bz * nt.x * nt.y;
-        const int by = rem / nt.x, bx = rem - by * nt.x;
-        float acc[VY];
-#pragma unroll
-        for (int v = 0; v < VY; ++v) acc[v] = 0.0f;
-        const int b1 = P.beam0 + P.n_beams;
-        for (int b = P.beam0; b < b1; ++b) {
-            __syncthreads();  // the previous beam's record no longer in use
-            pb_stage_record(&s_beam, beams + b, tid, kPbThreadsX * TY);
-            __syncthreads();
-            PbExtra x;
-            x.mu = s_beam.mu;
-            pb_tile<kPbDose, TY, VY>(P.g, s_beam.f, s_beam.t, s_beam.wet, bx, by, bz, acc, x);
-        }
-#pragma unroll
-        for (int v = 0; v < VY; ++v) {
-            const int3 q = pb_tile_voxel<TY, VY>(bx, by, bz, v);
-            const long long u = (long long)q.x + (long long)P.g.nx * (q.y + (long long)P.g.ny * q.z);
-            if (q.x < P.g.nx && q.y < P.g.ny && q.z < P.g.nz && DC_IN_BOUNDS(u, P.g.n(), 23)) P.dose[u] = acc[v];
-        }
-    }
+__global__ void __launch_bounds__(kPbThreadsX *TY, 4)
+    pb_kernel(Grid g, Frame f, ProtonTables t, const float *__restrict__ wet_s, PbExtra x) {
+    pb_tile<kMode, TY, VY>(g, f, t, wet_s, blockIdx.x, blockIdx.y, blockIdx.z, x);
 }
 
 DC_BOUNDS_TAKE(take_bounds_proton)
 
 static size_t pb_smem(int lut_len) {
-    return 2 * kPbSpotChunk * sizeof(float4) + kPbSpotChunk * sizeof(float) + 3 * (size_t)lut_len * sizeof(float);
+    return 2 * kPbSpotChunk * sizeof(float4) + 3 * (size_t)lut_len * sizeof(float);
 }
 
 template <class K>
@@ -809,114 +644,28 @@ static void pb_attr(K kernel, size_t smem, int device, bool *done) {
 
 template <int kMode>
 static void pb_launch(DeviceContext &ctx, const char *name, const Grid &g, const Frame &f, const ProtonTables &t,
-                      const float *wet_s, float *dose, const PbExtra &x, cudaStream_t s) {
+                      const float *wet_s, const PbExtra &x, cudaStream_t s) {
     const size_t smem = pb_smem(t.lut_len);
     static bool attr_set[64] = {false};
     pb_attr(pb_kernel<kMode, kPbThreadsY, kPbVoxY>, smem, ctx.device, attr_set);
     dim3 block(kPbThreadsX, kPbThreadsY, 1);
     const int3 nt = pb_tiles<kPbThreadsY, kPbVoxY>(g);
-    // tiles x.tile_z0 .. tile_z1 - 1 along z (all of them by default)
-    const int z1 = x.tile_z1 < 0 ? nt.z : std::min(x.tile_z1, nt.z);
-    if (x.tile_z0 < 0 || x.tile_z0 >= z1) return;
-    dim3 grid((unsigned)nt.x, (unsigned)nt.y, (unsigned)(z1 - x.tile_z0));
+    dim3 grid((unsigned)nt.x, (unsigned)nt.y, (unsigned)nt.z);
     KernelTimer kt(ctx, name, s);
-    pb_kernel<kMode, kPbThreadsY, kPbVoxY><<<grid, block, smem, s>>>(g, f, t, wet_s, dose, x);
+    pb_kernel<kMode, kPbThreadsY, kPbVoxY><<<grid, block, smem, s>>>(g, f, t, wet_s, x);
     check_launch(name);
 }
-
-void launch_pencil_beam(DeviceContext &ctx, const Grid &g, const Frame &f, const ProtonTables &t,
-                        const float *wet_s, float *dose, cudaStream_t s, const float *mu_dev, int tile_z0,
-                        int tile_z1) {
-    PbExtra x;
-    x.mu = mu_dev;
-    x.tile_z0 = tile_z0;
-    x.tile_z1 = tile_z1;
-    pb_launch<kPbDose>(ctx, "pencil_beam", g, f, t, wet_s, dose, x, s);
-}
-
-int pencil_beam_tile_depth() { return PbTileShape<kPbThreadsY, kPbVoxY>::z; }
 
 void launch_pencil_beam_mode(DeviceContext &ctx, int mode, const Grid &g, const Frame &f, const ProtonTables &t,
                              const float *wet_s, const PbExtra &x, cudaStream_t s) {
     switch (mode) {
-        case kPbAdjoint: pb_launch<kPbAdjoint>(ctx, "pencil_beam_adjoint", g, f, t, wet_s, nullptr, x, s); break;
-        case kPbSpotMax: pb_launch<kPbSpotMax>(ctx, "pencil_beam_spotmax", g, f, t, wet_s, nullptr, x, s); break;
-        case kPbCount: pb_launch<kPbCount>(ctx, "pencil_beam_count", g, f, t, wet_s, nullptr, x, s); break;
+        case kPbSpotMax: pb_launch<kPbSpotMax>(ctx, "pencil_beam_spotmax", g, f, t, wet_s, x, s); break;
+        case kPbCount: pb_launch<kPbCount>(ctx, "pencil_beam_count", g, f, t, wet_s, x, s); break;
         case kPbFill:
             if (x.row_ptr == nullptr) throw Error(DC_ERR_VALUE, "the fill pass needs the row starts");
-            pb_launch<kPbCount>(ctx, "pencil_beam_fill", g, f, t, wet_s, nullptr, x, s);
+            pb_launch<kPbCount>(ctx, "pencil_beam_fill", g, f, t, wet_s, x, s);
             break;
-        default: throw Error(DC_ERR_VALUE, "unknown pencil-beam mode");
-    }
-}
-
-template <int kMode>
-static void pb_list_launch(DeviceContext &ctx, const char *name, const Grid &g, const Frame &f,
-                           const ProtonTables &t, const float *wet_s, const PbExtra &x, cudaStream_t s) {
-    if (x.n_list <= 0) return;
-    const size_t smem = pb_smem(t.lut_len);
-    static bool attr_set[64] = {false};
-    pb_attr(pb_list_kernel<kMode, kPbThreadsY, kPbVoxY>, smem, ctx.device, attr_set);
-    const int per_cta = kPbThreadsX * kPbThreadsY * kPbVoxY;
-    const unsigned blocks = (unsigned)((x.n_list + per_cta - 1) / per_cta);
-    KernelTimer kt(ctx, name, s);
-    pb_list_kernel<kMode, kPbThreadsY, kPbVoxY><<<blocks, dim3(kPbThreadsX, kPbThreadsY, 1), smem, s>>>(g, f, t,
-                                                                                                     wet_s, x);
-    check_launch(name);
-}
-
-void launch_pencil_beam_list(DeviceContext &ctx, int mode, const Grid &g, const Frame &f, const ProtonTables &t,
-                             const float *wet_s, const PbExtra &x, cudaStream_t s) {
-    switch (mode) {
-        case kPbDose: pb_list_launch<kPbDose>(ctx, "pencil_beam_list", g, f, t, wet_s, x, s); break;
-        case kPbAdjoint: pb_list_launch<kPbAdjoint>(ctx, "pencil_beam_list_adjoint", g, f, t, wet_s, x, s); break;
-        default: throw Error(DC_ERR_VALUE, "voxel-list mode is for the dose and the adjoint");
-    }
-}
-
-// Tile shapes of the batch kernel (threads along y, voxels per thread along y).
-static const int kPbVariants[][2] = {{8, 2}, {4, 2}, {8, 1}, {4, 4}};
-int pencil_beam_batch_variants() { return (int)(sizeof(kPbVariants) / sizeof(kPbVariants[0])); }
-void pencil_beam_batch_tile(int variant, int *ty, int *vy) {
-    *ty = kPbVariants[variant][0];
-    *vy = kPbVariants[variant][1];
-}
-long long pencil_beam_batch_tiles(int variant, const Grid &g) {
-    int3 n{};
-    switch (variant) {
-        case 0: n = pb_tiles<8, 2>(g); break;
-        case 1: n = pb_tiles<4, 2>(g); break;
-        case 2: n = pb_tiles<8, 1>(g); break;
-        case 3: n = pb_tiles<4, 4>(g); break;
-        default: throw Error(DC_ERR_VALUE, "unknown pencil-beam tile variant");
-    }
-    return (long long)n.x * n.y * n.z;
-}
-
-template <int TY, int VY>
-static void pb_batch_launch(DeviceContext &ctx, const PbBatchPlan *plans, const PbBatchBeam *beams,
-                            const int2 *items, int n_items, unsigned *next, int lut_len, cudaStream_t s) {
-    const size_t smem = pb_smem(lut_len);
-    static bool attr_set[64] = {false};
-    pb_attr(pb_batch_kernel<TY, VY>, smem, ctx.device, attr_set);
-    int sms = 0, per_sm = 0;
-    DC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
-    DC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pb_batch_kernel<TY, VY>, kPbThreadsX * TY, smem));
-    const int blocks = std::max(1, std::min(n_items, sms * std::max(per_sm, 1)));
-    DC_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned), s));
-    KernelTimer kt(ctx, "pencil_beam_batch", s);
-    pb_batch_kernel<TY, VY><<<blocks, dim3(kPbThreadsX, TY, 1), smem, s>>>(plans, beams, items, n_items, next);
-    check_launch("pb_batch_kernel");
-}
-
-void launch_pencil_beam_batch(DeviceContext &ctx, int variant, const PbBatchPlan *plans, const PbBatchBeam *beams,
-                              const int2 *items, int n_items, unsigned *next, int lut_len, cudaStream_t s) {
-    switch (variant) {
-        case 0: pb_batch_launch<8, 2>(ctx, plans, beams, items, n_items, next, lut_len, s); break;
-        case 1: pb_batch_launch<4, 2>(ctx, plans, beams, items, n_items, next, lut_len, s); break;
-        case 2: pb_batch_launch<8, 1>(ctx, plans, beams, items, n_items, next, lut_len, s); break;
-        case 3: pb_batch_launch<4, 4>(ctx, plans, beams, items, n_items, next, lut_len, s); break;
-        default: throw Error(DC_ERR_VALUE, "unknown pencil-beam tile variant");
+        default: throw Error(DC_ERR_VALUE, "unknown influence pass");
     }
 }
 
