@@ -11,6 +11,19 @@ namespace dc {
 // ---- radiological depth (dc_wet.cu) --------------------------------------
 void launch_wet_march(DeviceContext &ctx, const Grid &g, const Frame &f, cudaTextureObject_t density,
                       float *wet, cudaStream_t s);
+// Smoothing samples in the reference's order (direction-major): the nearest
+// voxel's index offset per axis and in the volume; `exact` has a bit per axis
+// on which float rounding decides and the kernel evaluates the reference's
+// expression instead.  reach: largest offset per axis; pow2: axes whose
+// spacing is a power of two.
+constexpr int kSmoothSamples = 54;
+struct WetSmoothTable {
+    long long lin[kSmoothSamples];
+    short dx[kSmoothSamples], dy[kSmoothSamples], dz[kSmoothSamples], exact[kSmoothSamples];
+    int n_exact, pow2, reach[3];
+};
+WetSmoothTable make_wet_smooth_table(const Grid &g, const Frame &f);
+void enqueue_wet_smooth(const Grid &g, const Frame &f, const float *wet, float *wet_s, cudaStream_t s);
 void launch_wet_smooth(DeviceContext &ctx, const Grid &g, const Frame &f, const float *wet, float *wet_s,
                        cudaStream_t s);
 

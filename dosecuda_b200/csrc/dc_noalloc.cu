@@ -40,12 +40,10 @@
 
 #include "../../include/dosecuda.h"
 #include "dc_common.cuh"
+#include "dc_kernels.cuh"
 #include "dc_runtime.cuh"
 
 namespace dc {
-
-// Reference smoothing kernel (dc_wet.cu), reused unchanged.
-__global__ void wet_smooth_kernel(Grid g, Frame f, const float *__restrict__ wet, float *__restrict__ wet_s);
 
 constexpr long long kNoAllocMaxVoxels = 4LL << 20;  // 4,194,304 voxels
 
@@ -226,8 +224,7 @@ extern "C" int dc_proton_raytrace_noalloc(int gpu_id, const float *rlsp_dev, int
         const dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 3) / 4), (unsigned)nz), block(32, 4, 1);
         wet_march_linear_kernel<<<grid, block, 0, s>>>(g, f, rlsp_dev, scratch);
         check_launch("wet_march_linear_kernel");
-        wet_smooth_kernel<<<grid, block, 0, s>>>(g, f, scratch, wet_out_dev);
-        check_launch("wet_smooth_kernel");
+        enqueue_wet_smooth(g, f, scratch, wet_out_dev, s);
     } catch (const Error &err) {
         return fail(err.code, err.what());
     }

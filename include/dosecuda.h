@@ -212,6 +212,16 @@ int dc_proton_raytrace(int gpu_id,
                        float vsadx, float vsady,
                        float *wet_out);
 
+/* The smoothing's 54 samples (six directions x 1..9 mm, direction-major) as
+ * (dx, dy, dz, exact): the sampled voxel's index offset from the voxel being
+ * smoothed, and a bit per axis (1, 2, 4) on which the offset is not constant
+ * and is evaluated per voxel.  offsets: 54 x 4 ints.  Host only (no GPU);
+ * src_dist = (VSADX + VSADY) / 2.  No counterpart in the reference. */
+int dc_wet_smooth_offsets(int nz, int ny, int nx, const float spacing[3],
+                          const float origin[3], const float iso[3],
+                          double gantry_deg, float couch_deg, float src_dist,
+                          int *offsets);
+
 int dc_proton_raytrace_dev(int gpu_id,
                            const float *rlsp_dev, int nz, int ny, int nx,
                            const float spacing[3], const float origin[3],
