@@ -142,6 +142,7 @@ enum PbMode { kPbDose = 0, kPbAdjoint = 1, kPbSpotMax = 2, kPbCount = 3, kPbFill
 // accesses since the last call, and cleared (debug builds; 0 otherwise).
 unsigned long long take_bounds_wet();
 unsigned long long take_bounds_photon();
+unsigned long long take_bounds_cccs();
 unsigned long long take_bounds_proton();
 unsigned long long take_bounds_pencil();
 unsigned long long take_bounds_basis();

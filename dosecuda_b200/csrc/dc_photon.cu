@@ -5,12 +5,7 @@
 // primary and scatter source occlusion by every MLC leaf pair (a product of
 // erf edges), the off-axis intensity/softening profile, the 12-bin spectrum
 // attenuated along the radiological depth, and the electron contamination.
-//
-// cccs_kernel restates cccKernel (IMRTClasses.cu:252-350) with kernelTilt
-// (:173-203): per voxel with TERMA > 0.01, for 6 zenith cones x 12 azimuths,
-// a backward recursive march from ray_length (cm) down to 0 in steps of one
-// voxel spacing, sampling TERMA and density (hardware trilinear), with the
-// cone direction tilted so that its axis points at the source.
+// The collapsed-cone superposition is in dc_cccs.cu.
 //
 // B200 design points:
 //  * TERMA and density are written as one float2 texel into the
@@ -27,14 +22,11 @@
 //    the previous pair's top edge, and open fields repeat the leaf x
 //    positions, so the scatter source (about 33 pairs in range) costs
 //    about one erf per pair instead of four.
-//  * The TERMA kernel applies the CCCS mask and lists the active voxels; the
-//    CCCS is a persistent grid-stride loop over that list, so every lane of
-//    every warp marches (masked voxels no longer idle lanes).
+//  * The TERMA kernel applies the CCCS mask and marks and lists the active
+//    voxels.
 //  * The 72 image-space cone directions, the per-cone step tables (the float
 //    sequence ray_length, ray_length - sp, ... >= 0 that sets each cone's
-//    sample count) and the cone coefficients are computed once per call and
-//    held in shared memory; per sample the kernel does 3 FMAs of position,
-//    one float2 texture fetch, one SFU exponential and the two recursions.
+//    sample count) and the cone coefficients are computed once per call.
 //  * The TERMA kernel maps threads to 32x4 voxel tiles (coalesced stores).
 #include <algorithm>
 #include <cmath>
@@ -218,7 +210,7 @@ __global__ void __launch_bounds__(128) head_kernel(Grid g, Frame f, PhotonParams
 // linear filtering returns the stored value unchanged.  It also applies the
 // CCCS mask (dose 0 where TERMA <= 0.01, IMRTClasses.cu:270-273): masked
 // voxels get their zero dose here, the others are appended to `active`
-// (warp-aggregated), so the CCCS runs on full warps of active voxels only.
+// (warp-aggregated) and set in `mask`, a bit per voxel (mask_words per row).
 // dose (or null) receives the zero of masked voxels; terma_out (or null) a
 // linear copy of the TERMA volume.  `head` holds head_kernel's factors.
 __global__ void __launch_bounds__(128) terma_kernel(Grid g, Frame f, PhotonParams P, const float *__restrict__ wet,
@@ -226,7 +218,8 @@ __global__ void __launch_bounds__(128) terma_kernel(Grid g, Frame f, PhotonParam
                                                     cudaTextureObject_t dens_tex, cudaSurfaceObject_t td_surf,
                                                     float *__restrict__ electron,
                                                     float *__restrict__ dose, float *__restrict__ terma_out,
-                                                    int *__restrict__ active, unsigned *__restrict__ n_active) {
+                                                    int *__restrict__ active, unsigned *__restrict__ n_active,
+                                                    unsigned *__restrict__ mask) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
@@ -261,6 +254,7 @@ __global__ void __launch_bounds__(128) terma_kernel(Grid g, Frame f, PhotonParam
     if (!act && dose && v_ok) dose[v] = 0.0f;
     const unsigned live = __activemask();
     const unsigned bal = __ballot_sync(live, act);
+    if (threadIdx.x == 0) mask[((long long)k * g.ny + j) * gridDim.x + blockIdx.x] = bal;  // a warp is a row's 32 voxels
     if (act) {
         const int lane = threadIdx.x & 31;
         const int leader = __ffs(bal) - 1;
@@ -288,145 +282,6 @@ __global__ void cone_dirs_kernel(Frame f, CccsCones C, float4 *__restrict__ dirs
     const float3 th_head = make_float3(sth * cj, sth * sj, cth);
     const float3 t = head_to_image<true>(f, th_head);
     dirs[d] = make_float4(t.x, t.y, t.z, sth);
-}
-
-// ---------------------------------------------------------------------------
-// CCCS
-// ---------------------------------------------------------------------------
-// td_tex: float2 (TERMA, density) texture, border (0, AIR_DENSITY) — one
-// filtered fetch serves both of the reference's textures (the same
-// coordinates and weights apply to both channels).
-// Persistent grid-stride loop over the active voxels listed by the TERMA
-// kernel (every lane of a warp does a full 72-direction march).
-__device__ __forceinline__ float cccs_voxel(const Grid &g, const Frame &f, const CccsCones &C, float sp_cm,
-                                            const float4 *s_dir, const float *s_rl10, cudaTextureObject_t td_tex,
-                                            float3 p);
-
-__global__ void __launch_bounds__(128) cccs_kernel(Grid g, Frame f, CccsCones C, float sp_cm, float dose_scale,
-                                                   const float4 *__restrict__ dirs, cudaTextureObject_t td_tex,
-                                                   const float *__restrict__ electron, const int *__restrict__ active,
-                                                   const unsigned *__restrict__ n_active, float *__restrict__ dose) {
-    __shared__ float4 s_dir[kMaxCones * 12];
-    __shared__ float s_rl10[kMaxConeSteps];
-    const int tid = threadIdx.x;
-    for (int q = tid; q < C.n_cones * 12; q += blockDim.x) s_dir[q] = dirs[q];
-    for (int q = tid; q < C.total_steps; q += blockDim.x) s_rl10[q] = C.rl10[q];
-    __syncthreads();
-
-    const unsigned n = *n_active;
-    const int plane = g.nx * g.ny;
-    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int v = DC_IN_BOUNDS(t, g.n(), 13) ? __ldg(active + t) : -1;
-        if (!DC_IN_BOUNDS(v, g.n(), 13)) continue;
-        const int k = v / plane;
-        const int rem = v - k * plane;
-        const int j = rem / g.nx;
-        const int i = rem - j * g.nx;
-        const float3 p = voxel_xyz(g, f, i, j, k);
-        float dose_value = cccs_voxel(g, f, C, sp_cm, s_dir, s_rl10, td_tex, p);
-        dose_value += __ldg(electron + v);
-        dose[v] = (!isnan(dose_value) && dose_value >= 0.0f) ? dose_scale * dose_value : 0.0f;  // v checked above
-    }
-}
-
-// CCCS at an arbitrary list of voxels (the surrogate's probe): the same
-// per-voxel sum as cccs_kernel, with the mask taken from the TERMA texel.
-__global__ void __launch_bounds__(128) cccs_points_kernel(Grid g, Frame f, CccsCones C, float sp_cm, float dose_scale,
-                                                          const float4 *__restrict__ dirs, cudaTextureObject_t td_tex,
-                                                          const float *__restrict__ electron,
-                                                          const int *__restrict__ voxels, int n,
-                                                          float *__restrict__ out) {
-    __shared__ float4 s_dir[kMaxCones * 12];
-    __shared__ float s_rl10[kMaxConeSteps];
-    const int tid = threadIdx.x;
-    for (int q = tid; q < C.n_cones * 12; q += blockDim.x) s_dir[q] = dirs[q];
-    for (int q = tid; q < C.total_steps; q += blockDim.x) s_rl10[q] = C.rl10[q];
-    __syncthreads();
-    const int plane = g.nx * g.ny;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int v = __ldg(voxels + t);
-        if (v < 0 || (long long)v >= g.n()) {  // not a voxel of the grid
-            out[t] = 0.0f;
-            continue;
-        }
-        const int k = v / plane;
-        const int rem = v - k * plane;
-        const int j = rem / g.nx;
-        const int i = rem - j * g.nx;
-        const float T = tex3D<float2>(td_tex, (float)i + 0.5f, (float)j + 0.5f, (float)k + 0.5f).x;
-        float r = 0.0f;
-        if (!(T <= 0.01f)) {
-            const float3 p = voxel_xyz(g, f, i, j, k);
-            float dose_value = cccs_voxel(g, f, C, sp_cm, s_dir, s_rl10, td_tex, p);
-            dose_value += __ldg(electron + v);
-            r = (!isnan(dose_value) && dose_value >= 0.0f) ? dose_scale * dose_value : 0.0f;
-        }
-        out[t] = r;
-    }
-}
-
-// Sum over the 6 zenith cones x 12 azimuths of the backward recursion
-// (IMRTClasses.cu:289-339) for the voxel at image position p.
-__device__ __forceinline__ float cccs_voxel(const Grid &g, const Frame &f, const CccsCones &C, float sp_cm,
-                                            const float4 *s_dir, const float *s_rl10, cudaTextureObject_t td_tex,
-                                            float3 p) {
-    // kernelTilt (IMRTClasses.cu:173-203): rotate each direction by the
-    // rotation taking the central axis (iso -> source) onto voxel -> source.
-    const float3 uvec = unit_to_source(f, p);
-    const float3 axis0 = unit_to_source(f, make_float3(0.f, 0.f, 0.f));
-    const float costh = axis0.x * uvec.x + axis0.y * uvec.y + axis0.z * uvec.z;
-    const float3 ax = make_float3(axis0.y * uvec.z - axis0.z * uvec.y, axis0.z * uvec.x - axis0.x * uvec.z,
-                                  axis0.x * uvec.y - axis0.y * uvec.x);
-    const float inv1c = 1.0f / (1.0f + costh);
-    // A sample at distance 0 lies on the voxel centre whatever the direction
-    // (fmaf(r, 0, p) == p), so every cone whose sample distances end exactly
-    // at 0 fetches the same texel there: fetched once here and reused,
-    // which gives the same value as the 72 separate fetches.
-    const float3 tc0 = tex_coord(g, f, p);
-    const float2 td0 = tex3D<float2>(td_tex, tc0.x, tc0.y, tc0.z);
-
-    float dose_value = 0.0f;
-    for (int c = 0; c < C.n_cones; ++c) {
-        const float Am = C.Am[c], am = C.am[c], Bm = C.Bm[c], bm = C.bm[c];
-        const float nam_l2e = -am * kLog2e;
-        const int s0 = C.step_off[c], ns = C.n_steps[c];
-        for (int az = 0; az < 12; ++az) {
-            const float4 dv = s_dir[c * 12 + az];
-            const float sinth = dv.w;
-            const float cp = sinth * (Am / (am * am));
-            const float cs = sinth * (Bm / bm);
-            // Rodrigues: r = ax x v + v cos + ax (ax.v)/(1+cos)
-            float3 r;
-            r.x = ax.y * dv.z - ax.z * dv.y;
-            r.y = ax.z * dv.x - ax.x * dv.z;
-            r.z = ax.x * dv.y - ax.y * dv.x;
-            r.x += dv.x * costh;
-            r.y += dv.y * costh;
-            r.z += dv.z * costh;
-            const float sc = (ax.x * dv.x + ax.y * dv.y + ax.z * dv.z) * inv1c;
-            r.x += ax.x * sc;
-            r.y += ax.y * sc;
-            r.z += ax.z * sc;
-
-            float Rp = 0.0f, Rs = 0.0f;
-            for (int s = 0; s < ns; ++s) {
-                const float rl10 = s_rl10[s0 + s];
-                float3 q;
-                q.x = fmaf(r.x, rl10, p.x);
-                q.y = fmaf(r.y, rl10, p.y);
-                q.z = fmaf(r.z, rl10, p.z);
-                const float3 tc = tex_coord(g, f, q);
-                const float2 td = rl10 == 0.0f ? td0 : tex3D<float2>(td_tex, tc.x, tc.y, tc.z);
-                const float Ti = td.x;
-                const float Di = fmaxf(td.y, kAirDensity) * sp_cm;
-                const float ex = fast_exp2(nam_l2e * Di);
-                Rp = Rp * ex + (Ti * cp * (1.0f - ex));
-                Rs = Rs * (1.0f - (bm * Di)) + (Ti * Di * cs);
-            }
-            dose_value += am * Rp + bm * Rs;
-        }
-    }
-    return dose_value;
 }
 
 // ---------------------------------------------------------------------------
@@ -518,15 +373,6 @@ void build_photon_params(const dc_photon_model &m, const dc_control_point &cp, f
     C.total_steps = off;
 }
 
-static unsigned cccs_blocks(const DeviceContext &ctx, long long work) {
-    // persistent grid: as many resident CTAs as fit on every SM
-    int sms = 0, per_sm = 0;
-    DC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
-    DC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cccs_kernel, 128, 0));
-    const long long want = (work + 127) / 128;
-    return (unsigned)std::max(1LL, std::min<long long>(want, (long long)sms * std::max(per_sm, 1)));
-}
-
 DC_BOUNDS_TAKE(take_bounds_photon)
 
 // WET (cm) below which the electron contamination term of terma_kernel is
@@ -576,28 +422,11 @@ void enqueue_terma(DeviceContext &ctx, const Grid &g, const Frame &f, const Phot
         KernelTimer kt(ctx, "terma", s);
         terma_kernel<<<vol_grid(g), dim3(32, 4, 1), 0, s>>>(g, f, P, w.wet, ctx.head.as<const float4>(), w.dens_tex,
                                                             w.td_surf, w.electron, dose_dev, terma_out, w.active,
-                                                            w.n_active);
+                                                            w.n_active, w.mask);
         check_launch("terma_kernel");
     }
     cone_dirs_kernel<<<1, kMaxCones * 12, 0, s>>>(f, C, w.dirs);
     check_launch("cone_dirs_kernel");
-}
-
-void enqueue_cccs(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
-                  float dose_scale, float *dose_dev, cudaStream_t s) {
-    KernelTimer kt(ctx, "cccs", s);
-    cccs_kernel<<<cccs_blocks(ctx, g.n()), 128, 0, s>>>(g, f, C, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex,
-                                                        w.electron, w.active, w.n_active, dose_dev);
-    check_launch("cccs_kernel");
-}
-
-void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
-                         float dose_scale, const int *voxels, int n, float *out, cudaStream_t s) {
-    if (n <= 0) return;
-    KernelTimer kt(ctx, "cccs_points", s);
-    cccs_points_kernel<<<cccs_blocks(ctx, n), 128, 0, s>>>(g, f, C, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex,
-                                                              w.electron, voxels, n, out);
-    check_launch("cccs_points_kernel");
 }
 
 void run_photon_pipeline(DeviceContext &ctx, const Grid &g, const Frame &f, const PhotonParams &P,
@@ -616,9 +445,10 @@ void run_photon_pipeline(DeviceContext &ctx, const Grid &g, const Frame &f, cons
     w.wet = static_cast<float *>(ctx.wet_raw.ensure((size_t)n * sizeof(float)));
     w.electron = static_cast<float *>(ctx.electron.ensure((size_t)n * sizeof(float)));
     w.dirs = static_cast<float4 *>(ctx.small.ensure(kMaxCones * 12 * sizeof(float4)));
-    char *act = static_cast<char *>(ctx.active.ensure(256 + (size_t)n * sizeof(int)));
+    char *act = static_cast<char *>(ctx.active.ensure(256 + (size_t)n * sizeof(int) + mask_bytes(g)));
     w.n_active = reinterpret_cast<unsigned *>(act);
     w.active = reinterpret_cast<int *>(act + 256);
+    w.mask = reinterpret_cast<unsigned *>(act + 256 + (size_t)n * sizeof(int));
     w.xlat = &ctx.xlat;
     w.depth_mode = ctx.photon_depth_mode;
     w.depth_stats = static_cast<unsigned *>(ctx.xstat.ensure(sizeof(unsigned)));

@@ -45,12 +45,18 @@ struct FluenceMap {
 void build_photon_params(const dc_photon_model &m, const dc_control_point &cp, float spacing_cm,
                          PhotonParams &P, CccsCones &C);
 
+// 32-voxel words per row of the CCCS voxel mask.
+__host__ __device__ inline int mask_words(int nx) { return (nx + 31) / 32; }
+inline size_t mask_bytes(const Grid &g) { return (size_t)g.nz * g.ny * mask_words(g.nx) * sizeof(unsigned); }
+
 // Device work buffers of one photon calculation.
 struct PhotonWork {
     float *wet = nullptr;          // radiological depth, n floats
     float *electron = nullptr;     // electron contamination, n floats
     unsigned *n_active = nullptr;  // number of CCCS voxels (device counter)
     int *active = nullptr;         // CCCS voxel list, n ints
+    unsigned *mask = nullptr;      // CCCS voxels as bits: nz * ny rows of mask_words(nx) words
+    DeviceBuffer *points = nullptr;  // scratch of enqueue_cccs_points
     float4 *dirs = nullptr;        // kMaxCones*12 image-frame cone directions
     cudaTextureObject_t dens_tex = 0;  // density, border AIR_DENSITY
     cudaSurfaceObject_t td_surf = 0;   // (TERMA, density) float2 array
@@ -74,7 +80,7 @@ void photon_head_fork(DeviceContext &ctx, const Grid &g, const Frame &f, const P
 // of every masked voxel, terma_out (or null) a linear TERMA copy.
 void enqueue_terma(DeviceContext &ctx, const Grid &g, const Frame &f, const PhotonParams &P, const CccsCones &C,
                    const PhotonWork &w, float *dose_dev, float *terma_out, cudaStream_t s);
-// CCCS of every active voxel listed by the last enqueue_terma.
+// CCCS of every voxel in the last enqueue_terma's mask (dc_cccs.cu).
 void enqueue_cccs(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
                   float dose_scale, float *dose_dev, cudaStream_t s);
 // CCCS at n listed voxels into out[0..n).

@@ -36,7 +36,7 @@ struct dc_photon_beam {
     float origin[3] = {0, 0, 0};
     VolumeArray density;
     VolumeArray td;
-    DeviceBuffer wet, electron, active, dirs, probe, xlat;
+    DeviceBuffer wet, electron, active, dirs, probe, xlat, points;
     // fluence mode: the unmodulated TERMA and electron term of the last
     // dc_photon_beam_terma, and the adjoint's scratch
     DeviceBuffer terma0, electron0, fl_h;
@@ -59,9 +59,11 @@ struct dc_photon_beam {
         const size_t n = (size_t)g.n();
         w.wet = static_cast<float *>(wet.ensure(n * sizeof(float)));
         w.electron = static_cast<float *>(electron.ensure(n * sizeof(float)));
-        char *act = static_cast<char *>(active.ensure(256 + n * sizeof(int)));
+        char *act = static_cast<char *>(active.ensure(256 + n * sizeof(int) + mask_bytes(g)));
         w.n_active = reinterpret_cast<unsigned *>(act);
         w.active = reinterpret_cast<int *>(act + 256);
+        w.mask = reinterpret_cast<unsigned *>(act + 256 + n * sizeof(int));
+        w.points = &points;
         w.dirs = static_cast<float4 *>(dirs.ensure(kMaxCones * 12 * sizeof(float4)));
         w.dens_tex = density.texture(kAirDensity);
         w.td_surf = td.surf;
@@ -76,6 +78,7 @@ struct dc_photon_beam {
         td.release();
         wet.release();
         xlat.release();
+        points.release();
         terma0.release();
         electron0.release();
         fl_h.release();
