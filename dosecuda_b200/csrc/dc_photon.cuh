@@ -91,9 +91,10 @@ void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, cons
 // beam's work set, for a following enqueue_cccs (dc_fluence.cu).
 void enqueue_fluence_modulate(DeviceContext &ctx, const Grid &g, const Frame &f, const FluenceMap &M,
                               const float *F, const float *T0, const float *E0, const PhotonWork &w, cudaStream_t s);
-// grad_F[beamlet] = d(sum_v grad_dose_v D_v)/dF (float64), with h (n floats)
-// as scratch for s K^T grad_dose; the work set's active list, directions and
+// grad_F[beamlet] = d(sum_v grad_dose_v D_v)/dF (float64), with h
+// (fluence_scratch_floats, 16-byte aligned) as scratch for s K^T grad_dose; the work set's active list, directions and
 // density channel must be those of the TERMA pass that produced T0, E0.
+size_t fluence_scratch_floats(const Grid &g);
 void enqueue_fluence_adjoint(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C,
                              const FluenceMap &M, float dose_scale, const float *T0, const float *E0,
                              const PhotonWork &w, const float *grad_dose, float *h, double *grad_F, cudaStream_t s);

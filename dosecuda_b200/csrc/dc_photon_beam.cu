@@ -450,7 +450,7 @@ int dc_photon_beam_fluence_adjoint(dc_photon_beam *b, const dc_fluence_map *map,
         cudaStream_t s = as_stream(stream);
         const PhotonWork w = b->work();
         const float *e0 = electron0(*b, s);
-        float *h = static_cast<float *>(b->fl_h.ensure((size_t)b->g.n() * sizeof(float)));
+        float *h = static_cast<float *>(b->fl_h.ensure(fluence_scratch_floats(b->g) * sizeof(float)));
         enqueue_fluence_adjoint(ctx, b->g, b->f, b->C, M, b->dose_scale, b->terma0.as<float>(), e0, w, grad_dose_dev,
                                 h, grad_fluence_dev, s);
     });
