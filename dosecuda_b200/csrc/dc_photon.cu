@@ -110,7 +110,6 @@ __device__ __forceinline__ float head_transmission(const PhotonParams &P, float3
     float trans = 0.0f;
     for (int q = q0; q < q1; ++q) {
         const float xl = P.mlc_xl[q], xr = P.mlc_xr[q];
-        if (xl == xr) continue;  // closed pair: exposed source X is exactly 0
         const float yb = P.mlc_yb[q], yt = P.mlc_yt[q];
         const float a1 = edge_arg(yb, p.y, div, kinv);
         const float a2 = edge_arg(yt, p.y, div, kinv);
@@ -122,6 +121,7 @@ __device__ __forceinline__ float head_transmission(const PhotonParams &P, float3
             cached_xl = xl;
             cached_xr = xr;
         }
+        if (cached_ex == 0.0f) continue;  // beside the leaves: adds exactly 0
         const float erf_b = (yb == cached_y) ? cached_erf_y : erff(a1);
         const float erf_t = erff(a2);
         cached_y = yt;
@@ -317,12 +317,29 @@ void build_photon_params(const dc_photon_model &m, const dc_control_point &cp, f
     P.efd = m.electron_fitted_dmax;
     // headTransmission's leaf projection to the isocentre plane (IMRTClasses.cu:122,130-134).
     const float mlc_scale = (m.primary_source_distance - m.mlc_distance) / m.primary_source_distance;
-    P.n_pairs = cp.n_mlc_pairs;
+    // A closed pair transmits exactly 0 and is left out.  Neighbouring pairs
+    // with the same leaf positions whose y edges meet (to 1e-5 mm: the two
+    // sides of an edge are rounded separately) are one opening: their y terms
+    // telescope, erf(t1) - erf(b1) + erf(t2) - erf(b2) = erf(t2) - erf(b1), so
+    // a square field of 20 leaves costs the kernel 4 erf instead of 23
+    // (128^3, 10 x 10 cm: head kernel 0.160 -> 0.051 ms).
+    P.n_pairs = 0;
     for (int q = 0; q < cp.n_mlc_pairs; ++q) {
-        P.mlc_yb[q] = (cp.mlc_y_offset[q] - 0.5f * cp.mlc_y_width[q]) * mlc_scale;
-        P.mlc_yt[q] = (cp.mlc_y_offset[q] + 0.5f * cp.mlc_y_width[q]) * mlc_scale;
-        P.mlc_xl[q] = cp.mlc_x1[q] * mlc_scale;
-        P.mlc_xr[q] = cp.mlc_x2[q] * mlc_scale;
+        const float yb = (cp.mlc_y_offset[q] - 0.5f * cp.mlc_y_width[q]) * mlc_scale;
+        const float yt = (cp.mlc_y_offset[q] + 0.5f * cp.mlc_y_width[q]) * mlc_scale;
+        const float xl = cp.mlc_x1[q] * mlc_scale, xr = cp.mlc_x2[q] * mlc_scale;
+        if (xl == xr) continue;
+        const int last = P.n_pairs - 1;
+        if (last >= 0 && P.mlc_xl[last] == xl && P.mlc_xr[last] == xr && std::fabs(yb - P.mlc_yt[last]) <= 1e-5f &&
+            yt >= yb && P.mlc_yt[last] >= P.mlc_yb[last]) {
+            P.mlc_yt[last] = yt;
+            continue;
+        }
+        P.mlc_yb[P.n_pairs] = yb;
+        P.mlc_yt[P.n_pairs] = yt;
+        P.mlc_xl[P.n_pairs] = xl;
+        P.mlc_xr[P.n_pairs] = xr;
+        ++P.n_pairs;
     }
     // Leaf-pair range search precondition (head_transmission): finite y
     // edges, bottom <= top within a pair, both ascending across pairs.
