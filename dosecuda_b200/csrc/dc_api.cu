@@ -54,7 +54,7 @@ void copy_host_to_array(VolumeArray &a, const float *src, int nz, int ny, int nx
 
 // WET march + smoothing with the RLSP volume already in ctx.density.
 void proton_raytrace_core(DeviceContext &ctx, const Grid &g, const Frame &f, float *wet_s_dev, cudaStream_t s) {
-    float *wet = static_cast<float *>(ctx.wet_raw.ensure((size_t)g.n() * sizeof(float)));
+    float *wet = static_cast<float *>(ctx.wet_raw.ensure(march_bytes(g)));
     // RLSP texture with border 0 (IMPTClasses.cu:292).
     launch_wet_march(ctx, g, f, ctx.density.texture(0.0f), wet, s);
     launch_wet_smooth(ctx, g, f, wet, wet_s_dev, s);

@@ -255,7 +255,7 @@ int dc_proton_batch_commit(dc_proton_batch *b) {
         }
         std::vector<PbBatchPlan> hplans;
         int beam0 = 0;
-        long long max_vox = 0;
+        size_t wet_bytes = 0;
         for (auto &p : b->plans) {
             PbBatchPlan P;
             P.g = p.g;
@@ -264,7 +264,7 @@ int dc_proton_batch_commit(dc_proton_batch *b) {
             P.n_beams = (int)p.beams.size();
             beam0 += P.n_beams;
             hplans.push_back(P);
-            max_vox = std::max(max_vox, p.g.n());
+            wet_bytes = std::max(wet_bytes, march_bytes(p.g));
         }
         void *db = b->d_beams.ensure(hbeams.size() * sizeof(PbBatchBeam));
         DC_CUDA(cudaMemcpy(db, hbeams.data(), hbeams.size() * sizeof(PbBatchBeam), cudaMemcpyHostToDevice));
@@ -287,7 +287,7 @@ int dc_proton_batch_commit(dc_proton_batch *b) {
         void *fp = b->first_tile.ensure(first.size() * sizeof(long long));
         DC_CUDA(cudaMemcpy(fp, first.data(), first.size() * sizeof(long long), cudaMemcpyHostToDevice));
         b->queue.ensure(sizeof(unsigned));
-        b->wet_raw.ensure((size_t)max_vox * sizeof(float));
+        b->wet_raw.ensure(wet_bytes);
         for (auto &p : b->plans) {
             std::unique_ptr<VolumeArray> a(new VolumeArray());
             a->ensure(p.g.nx, p.g.ny, p.g.nz, false);

@@ -9,6 +9,9 @@
 namespace dc {
 
 // ---- radiological depth (dc_wet.cu) --------------------------------------
+// Bytes of the WET buffer of a march: the volume and a map of its uniform
+// parts behind it.
+size_t march_bytes(const Grid &g);
 void launch_wet_march(DeviceContext &ctx, const Grid &g, const Frame &f, cudaTextureObject_t density,
                       float *wet, cudaStream_t s);
 // Smoothing samples in the reference's order (direction-major): the nearest

@@ -459,7 +459,7 @@ void run_photon_pipeline(DeviceContext &ctx, const Grid &g, const Frame &f, cons
     ctx.terma.ensure(g.nx, g.ny, g.nz, true, 2);
     w.td_tex = ctx.terma.texture(0.0f, kAirDensity);
     w.td_surf = ctx.terma.surf;
-    w.wet = static_cast<float *>(ctx.wet_raw.ensure((size_t)n * sizeof(float)));
+    w.wet = static_cast<float *>(ctx.wet_raw.ensure(march_bytes(g)));
     w.electron = static_cast<float *>(ctx.electron.ensure((size_t)n * sizeof(float)));
     w.dirs = static_cast<float4 *>(ctx.small.ensure(kMaxCones * 12 * sizeof(float4)));
     char *act = static_cast<char *>(ctx.active.ensure(256 + (size_t)n * sizeof(int) + mask_bytes(g)));

@@ -57,7 +57,7 @@ struct dc_photon_beam {
     PhotonWork work() {
         PhotonWork w;
         const size_t n = (size_t)g.n();
-        w.wet = static_cast<float *>(wet.ensure(n * sizeof(float)));
+        w.wet = static_cast<float *>(wet.ensure(march_bytes(g)));
         w.electron = static_cast<float *>(electron.ensure(n * sizeof(float)));
         char *act = static_cast<char *>(active.ensure(256 + n * sizeof(int) + mask_bytes(g)));
         w.n_active = reinterpret_cast<unsigned *>(act);

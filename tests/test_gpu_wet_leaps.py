@@ -1,0 +1,44 @@
+"""WET march over uniform density (dc_wet.cu): samples added without a fetch."""
+import types
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape,spacing,gantry,couch", [
+    ((97, 101, 103), (2.0, 2.0, 2.0), 0.0, 0.0),     # axis-aligned; one voxel beyond whole bricks of 4 (x, z)
+    ((96, 128, 104), (2.5, 2.0, 1.5), 213.0, 25.0),  # whole bricks and tiles of 8 bricks, oblique
+    ((35, 260, 131), (3.0, 1.2, 3.1), 90.0, 0.0),    # thin along z, odd sizes
+])
+def test_leaps_equal_the_sampled_march(shape, spacing, gantry, couch):
+    """A volume in uniform pieces against the same volume with every voxel of
+    water or bone moved by one unit in the last place in a checkerboard, of
+    which no brick can be leapt over.  The moved values and the roundings of at
+    most 512 additions change a depth by less than 512 x 2^-23 of it."""
+    import torch
+
+    from dosecuda_b200 import engine
+
+    rng = np.random.default_rng(sum(shape))
+    nz, ny, nx = shape
+    rho = np.ones(shape, np.float32)
+    rho[:, : ny // 7, :] = 0.0                                      # air, with an exact zero
+    rho[nz // 3: nz // 3 + 9, ny // 2: ny // 2 + 14, 5: nx - 30] = 1.62
+    rho[nz // 2:, ny // 3: ny // 3 + 21, nx // 2:] = 0.26
+    rho[nz // 4: nz // 4 + 6, :, nx // 3: nx // 3 + 11] = -0.4      # counts as none
+    rho[:, ny - 20: ny - 11, 3: 20] += rng.uniform(-0.1, 0.1, (nz, 9, 17)).astype(np.float32)
+    odd = np.indices(shape).sum(0) % 2 == 1
+    moved = np.where(odd & (rho > 0), np.nextafter(rho, np.float32(2)), rho).astype(np.float32)
+
+    grid = types.SimpleNamespace(spacing=np.array(spacing), origin=np.array([-n * s / 2 for n, s in zip((nx, ny, nz), spacing)]))
+    beam = types.SimpleNamespace(iso=np.array([3.0, -7.0, 11.0], np.float32), gantry_angle=gantry, couch_angle=couch)
+    model = types.SimpleNamespace(VSADX=2000.0, VSADY=1800.0)
+    wet = [engine.proton_wet(torch.as_tensor(v, device="cuda"), grid, beam, model).cpu().numpy() for v in (rho, moved)]
+    deep = wet[1] > 1.1
+    assert deep.mean() > 0.5
+    # the number of voxels averaged steps with the unsmoothed depth below 1 cm, which is not seen
+    # here: a few voxels beside an edge stand on such a step and move with the last place
+    far = np.abs(wet[0] - wet[1])[deep] > 512 * 2.0 ** -23 * wet[1][deep]
+    assert far.mean() < 1e-5
