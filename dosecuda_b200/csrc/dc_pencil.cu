@@ -227,8 +227,9 @@ __device__ __forceinline__ void warp_beam(const ProtonTables &t, const PbExtra &
     for (int l0 = 0; l0 < t.n_layers; l0 += 32) {
         unsigned todo = layers_reaching(t, G, l0, wmin);
         for (; todo != 0u; todo &= todo - 1u) {
-            if (turn++ % step != first) continue;
             const int l = l0 + __ffs(todo) - 1;
+            // in turn over the tile's layers; a listed voxel's parts must not depend on which layers its warp reaches
+            if ((kList ? l : turn++) % step != first) continue;
             const LayerView L = load_layer(t.layers + l);
             const float r80 = L.r80;
             bool act[kVox];
@@ -491,54 +492,43 @@ __global__ void __launch_bounds__(32 * kWarps, 6)
     const long long e0 = ((long long)blockIdx.x * (kWarps / split) + tile) * kWarpVox;
     WarpGeom<true> G;
     float gv[kVox], acc[kVox];
-    const float3 ex = image_to_head<false>(f, make_float3(1.f, 0.f, 0.f));
-    const float3 ey = image_to_head<false>(f, make_float3(0.f, 1.f, 0.f));
-    const float3 ez = image_to_head<false>(f, make_float3(0.f, 0.f, 1.f));
     const long long plane = (long long)g.nx * g.ny;
-    long long vox[kVox];
-    long long ref = -1;  // reference voxel: a valid one near the middle of the warp's entries
-#pragma unroll
-    for (int q = 0; q < kVox; ++q) {
-        const int v = (q & 1) ? kVox / 2 - 1 - q / 2 : kVox / 2 + q / 2;
-        const long long e = e0 + v * 32 + lane;
-        const long long vi = e < x.n_list ? (long long)__ldg(x.list + e) : -1;
-        vox[v] = vi < plane * g.nz ? vi : -1;  // out-of-grid entries give 0
-        const unsigned m = __ballot_sync(0xffffffffu, vox[v] >= 0);
-        if (ref < 0 && m) ref = __shfl_sync(0xffffffffu, vi, v < kVox / 2 ? 31 - __clz(m) : __ffs(m) - 1);
-    }
-    const bool have = ref >= 0;
-    if (!have) ref = 0;
-    const int rk = (int)(ref / plane), rj = (int)((ref - rk * plane) / g.nx), ri = (int)(ref - rk * plane - (long long)rj * g.nx);
+    // Offsets are taken from the isocentre, not from a voxel of the warp: a
+    // voxel's distances then do not depend on the list's other entries.
+    G.c = make_float3(0.f, 0.f, 0.f);
+    G.cl = make_float2(0.f, 0.f);
+    G.dz = make_float3(0.f, 0.f, 0.f);
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    bool have = false;
 #pragma unroll
     for (int v = 0; v < kVox; ++v) {
         const long long e = e0 + v * 32 + lane;
-        const bool valid = vox[v] >= 0;
-        const long long u = valid ? vox[v] : 0;
+        const long long vi = e < x.n_list ? (long long)__ldg(x.list + e) : -1;
+        const bool valid = vi >= 0 && vi < plane * g.nz;  // out-of-grid entries give 0
+        const long long u = valid ? vi : 0;
         const int k = (int)(u / plane);
         const long long rem = u - (long long)k * plane;
         const int j = (int)(rem / g.nx), i = (int)(rem - (long long)j * g.nx);
-        const float ox = (float)(i - ri) * g.sx, oy = (float)(j - rj) * g.sy, oz = (float)(k - rk) * g.sz;
-        G.l[v] = make_float3(fmaf(ex.x, ox, fmaf(ey.x, oy, ez.x * oz)), fmaf(ex.y, ox, fmaf(ey.y, oy, ez.y * oz)),
-                             fmaf(ex.z, ox, fmaf(ey.z, oy, ez.z * oz)));
+        const float3 p = voxel_xyz(g, f, i, j, k);
+        G.l[v] = image_to_head<false>(f, p);
         G.wet[v] = INFINITY;
         G.dw[v] = 0.0f;
         gv[v] = 0.0f;
         acc[v] = 0.0f;
         if (valid && DC_IN_BOUNDS(u, g.n(), 21)) {
+            have = true;
             G.wet[v] = __ldg(wet_s + u) * 10.0f;
-            G.dw[v] = distance_to_source(f, voxel_xyz(g, f, i, j, k)) - G.wet[v];
+            G.dw[v] = distance_to_source(f, p) - G.wet[v];
             if (kAdj) gv[v] = __ldg(x.grad_dose + e);
             lo[0] = fminf(lo[0], G.l[v].x), hi[0] = fmaxf(hi[0], G.l[v].x);
             lo[1] = fminf(lo[1], G.l[v].y), hi[1] = fmaxf(hi[1], G.l[v].y);
             lo[2] = fminf(lo[2], G.l[v].z), hi[2] = fmaxf(hi[2], G.l[v].z);
         }
     }
-    head_centre(f, (double)ri * g.sx - f.isox, (double)rj * g.sy - f.isoy, (double)rk * g.sz - f.isoz, G.c, G.cl);
-    G.dz = make_float3(0.f, 0.f, 0.f);
-    G.bx0 = G.c.x + warp_min(lo[0]), G.bx1 = G.c.x + warp_max(hi[0]);
-    G.by0 = G.c.y + warp_min(lo[1]), G.by1 = G.c.y + warp_max(hi[1]);
-    G.bz0 = G.c.z + warp_min(lo[2]), G.bz1 = G.c.z + warp_max(hi[2]);
+    have = __any_sync(0xffffffffu, have);
+    G.bx0 = warp_min(lo[0]), G.bx1 = warp_max(hi[0]);
+    G.by0 = warp_min(lo[1]), G.by1 = warp_max(hi[1]);
+    G.bz0 = warp_min(lo[2]), G.bz1 = warp_max(hi[2]);
     if (have) warp_beam<kAdj, true>(t, x, G, mems[w], part, split, gv, acc);
     if (kAdj) return;
     if (split > 1) {
@@ -660,7 +650,7 @@ void list_launch(DeviceContext &ctx, const char *name, const Grid &g, const Fram
                  const float *wet_s, const PbExtra &x, cudaStream_t s) {
     if (x.n_list <= 0) return;
     const long long tiles = ((long long)x.n_list + kWarpVox - 1) / kWarpVox;
-    const int split = layer_split(ctx, tiles, t.n_layers);
+    const int split = layer_split(ctx, 0, t.n_layers);  // the same for every list, as a voxel's dose is
     const long long per = kWarps / split;
     constexpr size_t smem = kWarps * sizeof(WarpMem<kAdj>);
     KernelTimer kt(ctx, name, s);
