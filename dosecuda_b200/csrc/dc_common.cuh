@@ -117,6 +117,37 @@ __device__ __forceinline__ float3 unit_to_source(const Frame &f, float3 p) {
     return u;
 }
 
+// The ray march's sum, -0.05 + sum 0.1 max(rho, 0) over the samples p + t u,
+// t = 0, 1, 2, ... inside the texture box, by kLanes lanes of a warp per ray
+// (all lanes of the warp call it; `take` false: no ray): a lane fetches every
+// kLanes-th sample, kEach of them at once, and the values are added in the
+// order of t, so the sum is that of one thread walking the ray, bit for bit.
+// For passes too small to fill the chip with a thread per ray: there the
+// fetches' latency counts, not their rate.
+template <int kLanes, int kEach>
+__device__ __forceinline__ float march_lanes(const Grid &g, const Frame &f, cudaTextureObject_t density, float3 p,
+                                             float3 u, bool take) {
+    const int lane = threadIdx.x & (kLanes - 1);
+    float sum = -0.05f;
+    for (int t0 = 0;; t0 += kLanes * kEach) {
+        float r[kEach];
+        bool inside = false;
+#pragma unroll
+        for (int m = 0; m < kEach; ++m) {
+            const float t = (float)(t0 + m * kLanes + lane);
+            const float3 tc = tex_coord(g, f, make_float3(fmaf(u.x, t, p.x), fmaf(u.y, t, p.y), fmaf(u.z, t, p.z)));
+            inside = take && tex_inside(g, tc);
+            r[m] = inside ? fmaxf(tex3D<float>(density, tc.x, tc.y, tc.z), 0.0f) : 0.0f;
+        }
+#pragma unroll
+        for (int m = 0; m < kEach; ++m)
+#pragma unroll
+            for (int l = 0; l < kLanes; ++l) sum = fmaf(__shfl_sync(0xffffffffu, r[m], l, kLanes), 0.1f, sum);
+        // the inside samples are a prefix: a ray goes on while its batch's last lane is inside
+        if (!__any_sync(0xffffffffu, inside)) return sum;
+    }
+}
+
 __device__ __forceinline__ float distance_to_source(const Frame &f, float3 p) {
     return norm3df(f.srcx - p.x, f.srcy - p.y, f.srcz - p.z);
 }

@@ -9,11 +9,11 @@
 // the nearest-voxel WET at radii 1,2,.. mm (r < min(10*WET, 10)) along six
 // BEV directions.
 //
-// B200 mapping: one thread per voxel with a warp covering 32 consecutive x
-// voxels (coalesced loads/stores; the 32 rays of a warp march side by side so
-// their texture samples share cache lines), blocks of 32x4 voxels.  The march
-// is bound by the texture unit's trilinear fetch rate, one fetch per 1 mm
-// sample.  The smoothing adds 54 voxels at constant index offsets; see there.
+// B200 mapping: the march is bound by the texture unit's trilinear fetches,
+// one per 1 mm sample: by their latency in small volumes (wet_march_kernel,
+// eight lanes per ray), by their rate in larger ones, where samples in uniform
+// density are added without a fetch (wet_march_leap_kernel).  The smoothing
+// adds 54 voxels at constant index offsets; see there.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -27,38 +27,27 @@ namespace dc {
 
 DC_BOUNDS_WORD
 
+// March of the smaller volumes (march_leaps): eight lanes per ray, two samples
+// of each in flight; a block takes 16 voxels of a row.  Measured on B200 (us,
+// a thread per ray of 32 x 4 voxels per block -> eight lanes): 24^3 at 3 mm
+// 18.6 -> 11.3, 44 x 40 x 36 at 3 mm 24 -> 18.5, 56^3 at 2 mm 41 -> 32.5, 80^3 at
+// 2 mm 103 -> 92; in larger volumes the texture rate binds either way (127 x
+// 113 x 91 288 -> 318).  Four lanes of four samples are 2 us slower at 24^3 and
+// 1.5 us faster at 80^3.
+constexpr int kRayLanes = 8, kRayEach = 2;
 __global__ void __launch_bounds__(128) wet_march_kernel(Grid g, Frame f, cudaTextureObject_t density,
                                                         float *__restrict__ wet) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny) return;
-
+    const int i = blockIdx.x * (128 / kRayLanes) + threadIdx.x / kRayLanes, j = blockIdx.y, k = blockIdx.z;
     const float3 p = voxel_xyz(g, f, i, j, k);
     const float3 u = unit_to_source(f, p);
-
-    float wet_sum = -0.05f;
-    float t = 0.0f;
-    // The samples inside the volume form a prefix of t = 0,1,2,... (each
-    // coordinate is monotonic in t), so the loop stops at the first exit.
-    while (true) {
-        float3 q;
-        q.x = fmaf(u.x, t, p.x);
-        q.y = fmaf(u.y, t, p.y);
-        q.z = fmaf(u.z, t, p.z);
-        const float3 tc = tex_coord(g, f, q);
-        if (!tex_inside(g, tc)) break;
-        const float rho = tex3D<float>(density, tc.x, tc.y, tc.z);
-        wet_sum = fmaf(fmaxf(rho, 0.0f), 0.1f, wet_sum);
-        t += 1.0f;
-    }
+    const float sum = march_lanes<kRayLanes, kRayEach>(g, f, density, p, u, i < g.nx);
     const long long v = (long long)i + (long long)g.nx * (j + (long long)g.ny * k);
-    if (DC_IN_BOUNDS(v, g.n(), 1)) wet[v] = wet_sum;
+    if (i < g.nx && threadIdx.x % kRayLanes == 0 && DC_IN_BOUNDS(v, g.n(), 1)) wet[v] = sum;
 }
 
-// Uniform density leapt over.  The march above is bound by the texture
-// unit (1.9 trilinear samples per clock and SM, one per mm of ray).  Where all
-// eight voxels of a sample hold the same number c the filter returns exactly c
+// Uniform density leapt over, in the larger volumes.  A plain march is bound by
+// the texture unit (1.9 trilinear samples per clock and SM, one per mm of ray).
+// Where all eight voxels of a sample hold one number c the filter returns c
 // (its weights are multiples of 1/256 that add up to 1), so such a sample
 // needs no fetch: phantoms, the air around a patient, structures overridden to
 // one density.  A map of bricks of kBrick^3 voxels holds each brick's value
@@ -481,10 +470,11 @@ size_t march_bytes(const Grid &g) {
     return (size_t)g.n() * sizeof(float) + (size_t)B.nx * B.ny * B.nz * (sizeof(float) + 1);
 }
 
-// Whether the march leaps.  The map takes 14 to 45 us; a march shorter than
-// some 60 us (4e7 samples, a voxel's mean path being half the volume's mean
-// extent) could win little from it: 44 x 40 x 36 at 3 mm takes 25 us without,
-// 14 + 9 with where all is uniform and 14 + 29 where nothing is.
+// Whether the march leaps.  The map takes 14 to 45 us, so a march shorter than
+// some 90 us (4e7 samples, a voxel's mean path being half the volume's mean
+// extent) would win little and lose more where nothing is uniform: 80^3 at 2 mm
+// takes 92 us with eight lanes per ray; leaping 15 + 25 where all is uniform
+// and 15 + 104 where nothing is.
 static bool march_leaps(const Grid &g) {
     const double mean = (g.nx * (double)g.sx + g.ny * (double)g.sy + g.nz * (double)g.sz) / 6.0;  // mm to the boundary
     return (double)g.n() * mean > 4.0e7;
@@ -517,8 +507,8 @@ void launch_wet_march(DeviceContext &ctx, const Grid &g, const Frame &f, cudaTex
         return;
     }
     KernelTimer kt(ctx, "wet_march", s);
-    const dim3 grid((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 3) / 4), (unsigned)g.nz);
-    wet_march_kernel<<<grid, dim3(32, 4, 1), 0, s>>>(g, f, density, wet);
+    const dim3 grid((unsigned)((g.nx + 128 / kRayLanes - 1) / (128 / kRayLanes)), (unsigned)g.ny, (unsigned)g.nz);
+    wet_march_kernel<<<grid, 128, 0, s>>>(g, f, density, wet);
     check_launch("wet_march_kernel");
 }
 
