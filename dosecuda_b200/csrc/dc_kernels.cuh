@@ -50,8 +50,8 @@ struct XrayLattice {
 // apply (source inside or next to the volume, lattice too large).
 bool plan_xray_lattice(const Grid &g, const Frame &f, XrayLattice &L);
 // Photon WET (cm) of every voxel through the lattice, with the reference's
-// march for the voxels the lattice cannot serve (listed in list/n_list, which
-// need room for every voxel); the plain march when the lattice does not apply.
+// march for the voxels the lattice cannot serve (listed in list, which needs
+// room for every voxel; *n_list must be 0 on s); the plain march when the lattice does not apply.
 // Voxels whose WET comes out below `wet_exact` (cm) are marched exactly too
 // where their lattice rays disagree (+infinity: the plain march for every
 // voxel).  `stats` (device word, or

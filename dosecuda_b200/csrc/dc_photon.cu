@@ -173,11 +173,18 @@ float photon_erf_skip_bound() { return kErfSaturated; }
 // softening (offAxisFactors, IMRTClasses.cu:152-171), as (tp, ts, oaf, soft).
 // Split from the TERMA kernel so that it can run on a side stream while the
 // density is uploaded or the radiological depth is traced.
-__global__ void __launch_bounds__(128) head_kernel(Grid g, Frame f, PhotonParams P, float4 *__restrict__ head) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny) return;
+//
+// Bound by the error functions of the leaf edges in reach.  A warp takes 8 x 4
+// voxels, not a row of 32: it spans a quarter of the leaves' and openings'
+// edges, so its lanes agree more often on which pairs they reach.  B200 (us):
+// oblique 143 x 131 x 97, unequal leaves 241 -> 215; 128^3, unequal leaves 209
+// -> 195, open field 51 -> 48.
+constexpr int kHeadX = 8, kHeadY = 4, kHeadZ = 4;
+__global__ void __launch_bounds__(kHeadX * kHeadY * kHeadZ) head_kernel(Grid g, Frame f, PhotonParams P,
+                                                                              float4 *__restrict__ head) {
+    const int i = blockIdx.x * kHeadX + threadIdx.x, j = blockIdx.y * kHeadY + threadIdx.y;
+    const int k = blockIdx.z * kHeadZ + threadIdx.z;
+    if (i >= g.nx || j >= g.ny || k >= g.nz) return;
     const long long v = (long long)i + (long long)g.nx * (j + (long long)g.ny * k);
 
     const float3 p = voxel_xyz(g, f, i, j, k);
@@ -404,19 +411,25 @@ static float electron_exact_wet(const PhotonParams &P) {
     return INFINITY;
 }
 
+// Stream of the work beside the depth pass.  With the kernel profiler on it
+// runs on s itself, so that no kernel's timed interval includes another's
+// share of the SMs.
+static cudaStream_t head_stream(const DeviceContext &ctx, cudaStream_t s) {
+    return ctx.profiling && !DeviceContext::capturing(s) ? s : ctx.side;
+}
+
 void photon_head_fork(DeviceContext &ctx, const Grid &g, const Frame &f, const PhotonParams &P, cudaStream_t s) {
     float4 *head = static_cast<float4 *>(ctx.head.ensure((size_t)g.n() * sizeof(float4)));
-    // With the kernel profiler on, the head factors run on s itself, so that
-    // no kernel's timed interval includes another's share of the SMs.
-    const cudaStream_t hs = ctx.profiling && !DeviceContext::capturing(s) ? s : ctx.side;
+    const cudaStream_t hs = head_stream(ctx, s);
     DC_CUDA(cudaEventRecord(ctx.fork_ev, s));
     DC_CUDA(cudaStreamWaitEvent(hs, ctx.fork_ev, 0));
     {
         KernelTimer kt(ctx, "head", hs);
-        head_kernel<<<vol_grid(g), dim3(32, 4, 1), 0, hs>>>(g, f, P, head);
+        const dim3 grid((unsigned)((g.nx + kHeadX - 1) / kHeadX), (unsigned)((g.ny + kHeadY - 1) / kHeadY),
+                        (unsigned)((g.nz + kHeadZ - 1) / kHeadZ));
+        head_kernel<<<grid, dim3(kHeadX, kHeadY, kHeadZ), 0, hs>>>(g, f, P, head);
         check_launch("head_kernel");
     }
-    DC_CUDA(cudaEventRecord(ctx.join_ev, hs));
     ctx.head_forked = true;
 }
 
@@ -425,14 +438,20 @@ void enqueue_terma(DeviceContext &ctx, const Grid &g, const Frame &f, const Phot
     if (g.n() > 0x7fffffffLL) throw Error(DC_ERR_VALUE, "photon volumes are limited to 2^31 - 1 voxels.");
     // the head factors run beside the depth pass unless the caller forked them earlier
     if (!ctx.head_forked) photon_head_fork(ctx, g, f, P, s);
+    {
+        const cudaStream_t hs = head_stream(ctx, s);
+        cone_dirs_kernel<<<1, kMaxCones * 12, 0, hs>>>(f, C, w.dirs);
+        check_launch("cone_dirs_kernel");
+        DC_CUDA(cudaEventRecord(ctx.join_ev, hs));
+    }
+    DC_CUDA(cudaMemsetAsync(w.n_active, 0, 2 * sizeof(unsigned), s));  // and the depth pass's list
     if (w.depth_mode == 1 && w.xlat != nullptr)
-        launch_xray_depth(ctx, g, f, w.dens_tex, w.wet, w.active, w.n_active, *w.xlat, w.depth_stats,
+        launch_xray_depth(ctx, g, f, w.dens_tex, w.wet, w.active, w.n_active + 1, *w.xlat, w.depth_stats,
                           electron_exact_wet(P), s);  // the active list is free until the TERMA kernel fills it
     else {
         launch_wet_march(ctx, g, f, w.dens_tex, w.wet, s);
         if (w.depth_stats != nullptr) DC_CUDA(cudaMemsetAsync(w.depth_stats, 0xff, sizeof(unsigned), s));
     }
-    DC_CUDA(cudaMemsetAsync(w.n_active, 0, sizeof(unsigned), s));
     DC_CUDA(cudaStreamWaitEvent(s, ctx.join_ev, 0));
     ctx.head_forked = false;
     {
@@ -442,8 +461,6 @@ void enqueue_terma(DeviceContext &ctx, const Grid &g, const Frame &f, const Phot
                                                             w.n_active, w.mask);
         check_launch("terma_kernel");
     }
-    cone_dirs_kernel<<<1, kMaxCones * 12, 0, s>>>(f, C, w.dirs);
-    check_launch("cone_dirs_kernel");
 }
 
 void run_photon_pipeline(DeviceContext &ctx, const Grid &g, const Frame &f, const PhotonParams &P,

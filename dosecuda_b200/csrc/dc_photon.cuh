@@ -53,7 +53,7 @@ inline size_t mask_bytes(const Grid &g) { return (size_t)g.nz * g.ny * mask_word
 struct PhotonWork {
     float *wet = nullptr;          // radiological depth, n floats
     float *electron = nullptr;     // electron contamination, n floats
-    unsigned *n_active = nullptr;  // number of CCCS voxels (device counter)
+    unsigned *n_active = nullptr;  // number of CCCS voxels, then of the depth pass's marched voxels (device counters)
     int *active = nullptr;         // CCCS voxel list, n ints
     unsigned *mask = nullptr;      // CCCS voxels as bits: nz * ny rows of mask_words(nx) words
     DeviceBuffer *points = nullptr;  // scratch of enqueue_cccs_points
@@ -68,8 +68,9 @@ struct PhotonWork {
 
 // Enqueues the density-independent head factors of every voxel (collimator
 // transmission, off-axis factors) on the context's side stream, after the
-// work enqueued on s so far.  The next enqueue_terma joins it; without this
-// call enqueue_terma forks it itself, beside the depth pass.
+// work enqueued on s so far.  The next enqueue_terma adds the cone directions
+// there and joins it; without this call enqueue_terma forks it itself, beside
+// the depth pass.
 // Head-transmission skip bound check: the largest float x in [lo, hi] whose
 // device erff(+-x) is not exactly +-1 (0 when there is none; synchronous,
 // current device), and the bound the head kernel skips leaf pairs beyond.

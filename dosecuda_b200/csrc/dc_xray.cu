@@ -401,8 +401,9 @@ constexpr int kRayLanes = 8, kRayEach = 4;
 __global__ void __launch_bounds__(128) xray_fallback_kernel(Grid g, Frame f, cudaTextureObject_t density,
                                                             const int *__restrict__ list,
                                                             const unsigned *__restrict__ n_list,
-                                                            float *__restrict__ wet) {
+                                                            unsigned *__restrict__ stats, float *__restrict__ wet) {
     const unsigned n = *n_list;
+    if (stats != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *stats = n;
     const int plane = g.nx * g.ny;
     const int lanes = n < gridDim.x * blockDim.x / 2 ? kRayLanes : 1;
     const unsigned per = blockDim.x / lanes, stride = gridDim.x * per;
@@ -503,7 +504,6 @@ void launch_xray_depth(DeviceContext &ctx, const Grid &g, const Frame &f, cudaTe
         xray_lattice_kernel<<<grid, 32 * kRaysPerBlock, 0, s>>>(g, f, L, density, G);
         check_launch("xray_lattice_kernel");
     }
-    DC_CUDA(cudaMemsetAsync(n_list, 0, sizeof(unsigned), s));
     {
         KernelTimer kt(ctx, "xray_voxel", s);
         const dim3 grid((unsigned)((g.nx + 31) / 32), (unsigned)((g.ny + 3) / 4), (unsigned)g.nz);
@@ -517,10 +517,9 @@ void launch_xray_depth(DeviceContext &ctx, const Grid &g, const Frame &f, cudaTe
         DC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, xray_fallback_kernel, 128, 0));
         const long long want = (g.n() * kRayLanes + 127) / 128;
         const unsigned blocks = (unsigned)std::max(1LL, std::min<long long>(want, (long long)sms * std::max(per_sm, 1)));
-        xray_fallback_kernel<<<blocks, 128, 0, s>>>(g, f, density, list, n_list, wet);
+        xray_fallback_kernel<<<blocks, 128, 0, s>>>(g, f, density, list, n_list, stats, wet);
         check_launch("xray_fallback_kernel");
     }
-    if (stats != nullptr) DC_CUDA(cudaMemcpyAsync(stats, n_list, sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
 }
 
 }  // namespace dc
