@@ -1,0 +1,37 @@
+"""The fluence adjoint's scatter (dc_fluence.cu: pairs of voxels per 16-byte addition) on grids where pairs end
+at the volume's edge: one voxel along an axis, odd and even extents."""
+import types
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(1, 9, 2), (3, 5, 7), (6, 1, 33), (4, 8, 6)])
+def test_dose_and_adjoint_agree(shape):
+    """<g, dose(F)> = <adjoint(g), F>.  The dose's texture weights are rounded to 1/256 (half a unit, 1/512,
+    either way) while the adjoint's are not; on these grids most samples blend with the border's 0, so that
+    a sample may be off by 1/512 of itself: 2e-3 of the sum of |g| dose.  One voxel's part of the sum lost
+    or added elsewhere is larger than that."""
+    import torch
+
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTControlPoint, IMRTPlan
+
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    nz, ny, nx = shape
+    sp = 4.0
+    grid = types.SimpleNamespace(spacing=np.array([sp] * 3), origin=np.array([-n * sp / 2 for n in (nx, ny, nz)]))
+    rho = torch.ones(shape, device="cuda")
+    x12 = np.where(np.abs(model.mlc_offsets) <= 100.0, 90.0, 0.0)
+    mlc = np.array(np.vstack((-x12, x12, model.mlc_offsets, model.mlc_widths)), dtype=np.single).T
+    cp = IMRTControlPoint(np.array([0.0, 0.0, 0.0], np.single), 100.0, mlc, 30.0, 0.0, 15.0, None, None)
+    fb = engine.PhotonFluenceBeam.field_map(rho, grid, model, cp, pitch=30.0, margin=10.0)
+    gen = torch.Generator().manual_seed(2)
+    F = (torch.rand((fb.nb, fb.na), generator=gen) + 0.5).cuda()
+    dose = fb.dose(F).double()
+    for _ in range(4):
+        g = torch.randn(shape, generator=gen).cuda()
+        lhs, rhs = float((g.double() * dose).sum()), float((fb.adjoint(g).reshape(F.shape) * F.double()).sum())
+        assert abs(lhs - rhs) <= 2e-3 * float((g.double().abs() * dose).sum())
