@@ -838,7 +838,7 @@ def pencil_beam_roofline(r):
     """The pencil beam's roofline.  Work unit (the algorithmic count, from the
     oracle): a (voxel, spot) pair within the layer's range whose distance from
     the spot axis is inside 6 halo sigmas at that voxel, 20 FP32 flops and 2
-    SFU ex2 each.  The kernel culls spots per CTA, so it evaluates somewhat
+    SFU ex2 each.  The kernel culls spots per warp tile, so it evaluates somewhat
     more pairs than that; the dense count (every in-range voxel x every spot of
     the layer, the reference's work) is reported beside it."""
     sm_hz = r["pk"].get("sm_max_mhz", 1965.0) * 1e6
@@ -876,7 +876,8 @@ def stage_rates(prof, nvox, march_samples, fetch_rate):
             e.update({"samples": int(march_samples), "samples_per_s": round(rate, 1)})
             if fetch_rate:
                 e["texture_frac"] = round(rate / fetch_rate, 4)
-                e["texture_peak_kind"] = "measured float2 fetch rate (dc_texture_fetch_rate); the march fetches float"
+                e["texture_peak_kind"] = ("measured float2 fetch rate (dc_texture_fetch_rate); the march fetches float, "
+                                          "and adds samples in uniform density without a fetch")
         if name in ("wet_march", "wet_smooth"):
             e["hbm_gbs_compulsory"] = round(8.0 * nvox / (ms * 1e-3) / 1e9, 2)
         out[name] = e
@@ -947,10 +948,11 @@ def main_mine(args):
                            "array page-locked by the call)",
                     "pinned_input": {"value": round(r["e2e_pinned_ms"] / (r["n_e2e"] * ws), 4), "unit": "ms/beam",
                                      "what": "the same call with a page-locked input array"}},
-            # The CCCS's binding unit is the texture pipe (one filtered float2
-            # fetch per cone sample; L1TEX ~95 % busy under ncu), so the
-            # top-level roof is the fetch rate measured on this GPU by
-            # dc_texture_fetch_rate; FP32 and HBM fractions are given beside it.
+            # The CCCS's binding unit is the texture pipe, so the top-level roof
+            # is the fetch rate measured on this GPU by dc_texture_fetch_rate.
+            # About a quarter of the samples is interpolated from shared memory
+            # beside it, so the fraction can exceed 1.  FP32 and HBM fractions
+            # are given beside it.
             "roofline": {
                 "bound": "texture" if tex else "fp32",
                 "kernel": "cccs",
@@ -959,8 +961,8 @@ def main_mine(args):
                 "unit": "filtered float2 fetches/s" if tex else "TFLOP/s",
                 "frac": (tex or {}).get("frac", round(r["achieved_tf"] / r["fp32_peak"], 4)),
                 "peak_kind": (tex or {}).get("peak_kind", "nominal FP32"),
-                "work": f"{r['samples']} cone samples (oracle count), one filtered float2 fetch + 1 SFU exp + "
-                        f"~18 FP32 flops each",
+                "work": f"{r['samples']} cone samples (oracle count), one filtered float2 fetch (or its "
+                        f"value from shared memory) + 1 SFU exp + ~18 FP32 flops each",
                 "samples_per_s": round(r["samples"] / (r["cccs_avg_ms"] * 1e-3), 1),
                 "kernel_ms": round(r["cccs_avg_ms"], 4),
                 "fp32": {"achieved_tflops": round(r["achieved_tf"], 3), "peak_tflops": round(r["fp32_peak"], 2),

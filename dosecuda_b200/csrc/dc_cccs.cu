@@ -387,16 +387,18 @@ void enqueue_cccs(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsC
     cccs(ctx, g, f, C, w, dose_scale, w.mask, dose_dev, s);
 }
 
+size_t cccs_points_bytes(const Grid &g) {
+    return ((mask_bytes(g) + 255) & ~(size_t)255) + (size_t)g.n() * sizeof(float);
+}
+
 // The listed voxels go through the same kernel as the full volume, behind
 // their own mask, so their doses are the full calculation's bit for bit.
 void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
-                         float dose_scale, const int *voxels, int n, float *out, cudaStream_t s) {
+                         float dose_scale, const int *voxels, int n, float *out, void *scratch, cudaStream_t s) {
     if (n <= 0) return;
     const size_t mb = mask_bytes(g);
-    const size_t mask_al = (mb + 255) & ~(size_t)255;
-    char *buf = static_cast<char *>(w.points->ensure(mask_al + (size_t)g.n() * sizeof(float)));
-    unsigned *points = reinterpret_cast<unsigned *>(buf);
-    float *dose = reinterpret_cast<float *>(buf + mask_al);
+    unsigned *points = static_cast<unsigned *>(scratch);
+    float *dose = reinterpret_cast<float *>(static_cast<char *>(scratch) + ((mb + 255) & ~(size_t)255));
     KernelTimer kt(ctx, "cccs_points", s);
     DC_CUDA(cudaMemsetAsync(points, 0, mb, s));
     const unsigned blocks = (unsigned)((n + 127) / 128);

@@ -56,7 +56,6 @@ struct PhotonWork {
     unsigned *n_active = nullptr;  // number of CCCS voxels, then of the depth pass's marched voxels (device counters)
     int *active = nullptr;         // CCCS voxel list, n ints
     unsigned *mask = nullptr;      // CCCS voxels as bits: nz * ny rows of mask_words(nx) words
-    DeviceBuffer *points = nullptr;  // scratch of enqueue_cccs_points
     float4 *dirs = nullptr;        // kMaxCones*12 image-frame cone directions
     cudaTextureObject_t dens_tex = 0;  // density, border AIR_DENSITY
     cudaSurfaceObject_t td_surf = 0;   // (TERMA, density) float2 array
@@ -84,9 +83,10 @@ void enqueue_terma(DeviceContext &ctx, const Grid &g, const Frame &f, const Phot
 // CCCS of every voxel in the last enqueue_terma's mask (dc_cccs.cu).
 void enqueue_cccs(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
                   float dose_scale, float *dose_dev, cudaStream_t s);
-// CCCS at n listed voxels into out[0..n).
+// CCCS at n listed voxels into out[0..n); scratch: cccs_points_bytes.
+size_t cccs_points_bytes(const Grid &g);
 void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
-                         float dose_scale, const int *voxels, int n, float *out, cudaStream_t s);
+                         float dose_scale, const int *voxels, int n, float *out, void *scratch, cudaStream_t s);
 
 // Fluence-modulated TERMA (m*T0) and electron term (m*E0) of the photon
 // beam's work set, for a following enqueue_cccs (dc_fluence.cu).

@@ -347,7 +347,7 @@ class ProtonBatch:
     spot_list).  After ``commit()``, ``wet()`` computes every beam's WET and
     ``dose(mu)`` every plan's dose (``self.doses[plan_id]``); both only enqueue
     device work, so they can be captured with ``torch.cuda.CUDAGraph``.
-    ``autotune()`` times the kernel's tile shapes on this workload and keeps
+    ``autotune()`` times the kernel's block shapes on this workload and keeps
     the fastest (cached in a JSON file keyed by the workload and GPU)."""
 
     def __init__(self, model, device="cuda"):
@@ -487,7 +487,7 @@ class ProtonBatch:
         return row_ptr, col[:nnz.value], val[:nnz.value]
 
     def autotune(self, cache_path: str | None = None, repeats: int = 3) -> int:
-        """Time every tile shape of the batch dose kernel on this workload and
+        """Time every block shape of the batch dose kernel on this workload and
         keep the fastest; results are cached in ``cache_path`` (JSON)."""
         import json
         import os

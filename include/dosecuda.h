@@ -361,7 +361,7 @@ int dc_proton_batch_add_plan(dc_proton_batch *batch, int nz, int ny, int nx, con
 int dc_proton_batch_add_beam(dc_proton_batch *batch, int plan_id, const float iso[3], double gantry_deg,
                              float couch_deg, const float *spots, int n_spots, float *wet_dev, int *beam_id);
 int dc_proton_batch_commit(dc_proton_batch *batch);
-/* n_variants: tile shapes the dose call accepts (for autotuning). */
+/* n_variants: block shapes the dose call accepts (for autotuning). */
 int dc_proton_batch_info(const dc_proton_batch *batch, int *n_plans, int *n_beams, int *n_spots_total,
                          int *n_variants);
 /* Offset of a beam's spots in the batch's spot-weight vector. */
