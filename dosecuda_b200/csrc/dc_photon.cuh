@@ -83,10 +83,9 @@ void enqueue_terma(DeviceContext &ctx, const Grid &g, const Frame &f, const Phot
 // CCCS of every voxel in the last enqueue_terma's mask (dc_cccs.cu).
 void enqueue_cccs(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
                   float dose_scale, float *dose_dev, cudaStream_t s);
-// CCCS at n listed voxels into out[0..n); scratch: cccs_points_bytes.
-size_t cccs_points_bytes(const Grid &g);
+// CCCS at n listed voxels into out[0..n).
 void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsCones &C, const PhotonWork &w,
-                         float dose_scale, const int *voxels, int n, float *out, void *scratch, cudaStream_t s);
+                         float dose_scale, const int *voxels, int n, float *out, cudaStream_t s);
 
 // Fluence-modulated TERMA (m*T0) and electron term (m*E0) of the photon
 // beam's work set, for a following enqueue_cccs (dc_fluence.cu).

@@ -19,7 +19,6 @@
 #include <cmath>
 #include <cstring>
 #include <iterator>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -37,7 +36,7 @@ struct dc_photon_beam {
     float origin[3] = {0, 0, 0};
     VolumeArray density;
     VolumeArray td;
-    DeviceBuffer wet, electron, active, dirs, probe, xlat, points;
+    DeviceBuffer wet, electron, active, dirs, probe, xlat;
     // fluence mode: the unmodulated TERMA and electron term of the last
     // dc_photon_beam_terma, and the adjoint's scratch
     DeviceBuffer terma0, electron0, fl_h;
@@ -52,8 +51,6 @@ struct dc_photon_beam {
     bool have_density = false, have_terma = false;
     std::vector<int> probe_host;
     int lattice = 4;                  // probe lattice stride (0: lines only)
-    std::mutex points_mu;             // one probe is enqueued at a time:
-    cudaEvent_t points_ev = nullptr;  // the last one's use of `points`
     PinnedBuffer probe_pin;           // staging of the probe list
     cudaEvent_t probe_ev = nullptr;   // its last upload
 
@@ -80,7 +77,6 @@ struct dc_photon_beam {
         td.release();
         wet.release();
         xlat.release();
-        points.release();
         terma0.release();
         electron0.release();
         fl_h.release();
@@ -92,7 +88,6 @@ struct dc_photon_beam {
         dirs.release();
         probe.release();
         if (probe_ev) cudaEventSynchronize(probe_ev), cudaEventDestroy(probe_ev);
-        if (points_ev) cudaEventSynchronize(points_ev), cudaEventDestroy(points_ev);
         probe_pin.release();
     }
 };
@@ -512,27 +507,9 @@ int dc_photon_beam_probe(dc_photon_beam *b, const int *voxels_dev, int n, float 
         }
         need(n >= 0, "'n' must not be negative.");
         DC_CUDA(cudaSetDevice(b->device));
-        if (n == 0) return;
         DeviceContext &ctx = context(b->device);
-        cudaStream_t s = as_stream(stream);
-        const PhotonWork w = b->work();
-        const size_t bytes = cccs_points_bytes(b->g);
-        std::lock_guard<std::mutex> lk(b->points_mu);
-        if (DeviceContext::capturing(s)) {  // a graph may run beside other probes: scratch of its own
-            void *scratch = nullptr;
-            DC_CUDA(cudaMallocAsync(&scratch, bytes, s));
-            enqueue_cccs_points(ctx, b->g, b->f, b->C, w, b->dose_scale, voxels_dev, n, dose_out_dev, scratch, s);
-            DC_CUDA(cudaFreeAsync(scratch, s));
-            return;
-        }
-        // probes of this beam on several streams take turns on its scratch
-        if (b->points_ev)
-            DC_CUDA(cudaStreamWaitEvent(s, b->points_ev, 0));
-        else
-            DC_CUDA(cudaEventCreateWithFlags(&b->points_ev, cudaEventDisableTiming));
-        enqueue_cccs_points(ctx, b->g, b->f, b->C, w, b->dose_scale, voxels_dev, n, dose_out_dev,
-                            b->points.ensure(bytes), s);
-        DC_CUDA(cudaEventRecord(b->points_ev, s));
+        enqueue_cccs_points(ctx, b->g, b->f, b->C, b->work(), b->dose_scale, voxels_dev, n, dose_out_dev,
+                            as_stream(stream));
     });
 }
 

@@ -1,7 +1,7 @@
 """The tiled collapsed-cone kernel (dc_cccs.cu) where its split of the samples between the texture unit and
 shared memory, its tiles and its voxel mask can go wrong, against the CPU oracle with the texture unit's
 rounded axis fractions: grids one voxel past a tile, spacings that put 1 to 10 samples of a cone in shared
-memory, uneven spacings, both tile shapes, fields that leave tiles partly or wholly masked.
+memory, uneven spacings, fields that leave tiles partly or wholly masked.
 
 Tolerance: the oracle rounds the three fractions to 1/256 and multiplies them exactly; the hardware also
 rounds each of the eight products to 1/256 (half a unit, 1/512, each way).  A sample between texels that
@@ -19,12 +19,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape,spacing,gantry,couch,field", [
-    ((5, 9, 9), (2.5, 2.5, 2.5), 0.0, 0.0, 30.0),       # one voxel past a tile, small tiles
+    ((5, 9, 9), (2.5, 2.5, 2.5), 0.0, 0.0, 30.0),       # one voxel past a tile
     ((1, 1, 40), (2.0, 2.0, 2.0), 90.0, 0.0, 20.0),     # a single row
     ((30, 33, 41), (4.0, 4.0, 4.0), 37.0, 15.0, 60.0),  # few samples per cone
     ((24, 30, 28), (1.0, 1.0, 1.0), 200.0, 0.0, 12.0),  # many
     ((33, 40, 47), (2.5, 2.0, 3.0), 310.0, -20.0, 40.0),  # uneven spacings: the reach differs per axis
-    ((70, 90, 97), (3.0, 3.0, 3.0), 25.0, 0.0, 50.0),   # large tiles, most of them masked
+    ((70, 90, 97), (3.0, 3.0, 3.0), 25.0, 0.0, 50.0),   # most tiles masked
 ])
 def test_dose_vs_oracle(shape, spacing, gantry, couch, field):
     import oracle
