@@ -26,14 +26,14 @@
 //    and add the parts in a fixed order, so the result stays deterministic.
 //
 // Measured on B200 (ms; before = the 16 x 8 x 4 tile per block of 256 threads
-// with its per-layer barriers): 96^3 beam of 2034 spots 0.95 -> 0.43; oblique
-// 127 x 113 x 91 with range shifter, 2831 spots 1.08 -> 0.66; 256 x 256 x 160,
-// 2655 spots 2.32 -> 1.35; six beams of 160 x 160 x 96 in one batch 5.90 ->
-// 3.22; dose / adjoint at 105 k listed voxels, 6025 spots 0.48 -> 0.30 / 1.63
-// -> 0.32.  Of the batch's cycles the exponentials take 55 %, instruction issue
-// 67 % (half of it the per-layer parameters, spot tests and lists).  Fewer or
-// more registers (24 to 40 warps per SM) changed nothing above 1 %; evaluating
-// a quarter of the exponentials as polynomials on the FP32 pipe cost 5 %.
+// with its per-layer barriers): 96^3 beam of 2034 spots 0.95 -> 0.41; oblique
+// 127 x 113 x 91 with range shifter, 2831 spots 1.08 -> 0.62; 256 x 256 x 160,
+// 2655 spots 2.32 -> 1.27; six beams of 160 x 160 x 96 in one batch 5.90 ->
+// 2.83; dose / adjoint at 105 k listed voxels, 6025 spots 0.48 -> 0.29 / 1.63
+// -> 0.29.  Of the batch's cycles the exponentials take 62 %.  Fewer or more
+// registers (24 to 40 warps per SM) changed nothing above 1 %; evaluating a
+// quarter of the exponentials as polynomials on the FP32 pipe cost 5 %, tiles
+// of 8 x 4 x 8 voxels 4 to 15 %.
 #include <algorithm>
 #include <cmath>
 
@@ -395,6 +395,12 @@ __device__ __forceinline__ void warp_beam(const ProtonTables &t, const PbExtra &
     }
 }
 
+// The warp's index in its block through a shuffle, which lets the compiler see
+// that it is the same in all lanes: the addresses of the warp's shared memory
+// then live in uniform registers and cost the pair loops no instructions (batch
+// of six beams 3.24 -> 2.83 ms, 256 x 256 x 160 1.35 -> 1.27).
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
 // Geometry of the tile with low corner (i0, j0, k0) and, when a layer of the
 // beam comes near its box, the voxels' depths; false when none does.  gv: the
 // voxels' gradients where grad is given (0 outside the grid).
@@ -448,7 +454,7 @@ __global__ void __launch_bounds__(32 * kWarps, 7)
                        PbExtra x, int split) {
     extern __shared__ float4 smem4[];
     WarpMem<kAdj> *mems = reinterpret_cast<WarpMem<kAdj> *>(smem4);
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = warp_index(), lane = threadIdx.x & 31;
     const int tile = w / split, part = w - tile * split;
     const int bx = split == 4 ? 1 : 2, by = split == 1 ? 2 : 1;  // tiles of the block along x and y
     const int i0 = (blockIdx.x * bx + tile % bx) * kTileX, j0 = (blockIdx.y * by + tile / bx) * kTileY;
@@ -487,7 +493,7 @@ __global__ void __launch_bounds__(32 * kWarps, 6)
     pencil_list_kernel(Grid g, Frame f, ProtonTables t, const float *__restrict__ wet_s, PbExtra x, int split) {
     extern __shared__ float4 smem4[];
     WarpMem<kAdj> *mems = reinterpret_cast<WarpMem<kAdj> *>(smem4);
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = warp_index(), lane = threadIdx.x & 31;
     const int tile = w / split, part = w - tile * split;
     const long long e0 = ((long long)blockIdx.x * (kWarps / split) + tile) * kWarpVox;
     WarpGeom<true> G;
@@ -573,7 +579,7 @@ __global__ void __launch_bounds__(32 * kW, 28 / kW)
                         const long long *__restrict__ first_tile, int n_plans, unsigned *__restrict__ next) {
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31;
-    BatchMem &M = reinterpret_cast<BatchMem *>(smem4)[threadIdx.x >> 5];
+    BatchMem &M = reinterpret_cast<BatchMem *>(smem4)[warp_index()];
     const long long n_items = __ldg(first_tile + n_plans);
     while (true) {
         unsigned it = 0;
