@@ -40,8 +40,8 @@ PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # capture (its command and figures).  A kernel change makes its entry stale
 # until it is captured again.
 NCU_TRAFFIC = {
-    "cccs": (15107328, "profiles/cccs_photon_small.md"),
-    "pencil_beam": (3622912, "profiles/pencil_beam_proton_small.md"),
+    "cccs": (12782592, "profiles/cccs_photon_small.md"),
+    "pencil_beam": (4148480 + 50432, "profiles/pencil_beam_proton_small.md"),
     "conv_dec0": (67162880 + 26884352, "profiles/conv_gather_dec0_surrogate_128.md"),
 }
 SM_COUNT = 148

@@ -18,10 +18,9 @@
 //    exactly erf = +-1 on both edges (kErfSaturated), i.e. no transmission;
 //    they are skipped without evaluating erf, and with ascending leaf edges
 //    the pairs that remain form one range found by binary search.  Within
-//    it, erf values of equal arguments are reused: a pair's bottom edge is
-//    the previous pair's top edge, and open fields repeat the leaf x
-//    positions, so the scatter source (about 33 pairs in range) costs
-//    about one erf per pair instead of four.
+//    it, erf values of equal arguments are reused (a pair's bottom edge is
+//    the previous pair's top edge).  Closed pairs are dropped and equal
+//    neighbours merged into one opening on the host (build_photon_params).
 //  * The TERMA kernel applies the CCCS mask and marks and lists the active
 //    voxels.
 //  * The 72 image-space cone directions, the per-cone step tables (the float
