@@ -81,7 +81,7 @@ struct __align__(16) LayerRec {
     float lut_d0, lut_inv, lut_step;
     // device: coefficients of the nuclear halo's sigma (log and pole terms)
     // and weight (log argument, quotient, linear term) at this R80
-    float hs_log, hs_pole, hw_arg, hw_num, hw_den, hw_lin;
+    float hs_log, hs_pole, hw_arg, hw_num, hw_edge, hw_lin;
 };
 
 

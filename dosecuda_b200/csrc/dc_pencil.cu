@@ -76,7 +76,7 @@ struct VoxelLayer {
 
 // The special-function unit's forms without the denormal handling of
 // __fdividef and __log2f (several instructions each; none of the operands
-// here is denormal), and 1 / x to within an ulp with one Newton step.
+// here is denormal).
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -87,15 +87,11 @@ __device__ __forceinline__ float log2_approx(float x) {
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float recip(float x) {
-    const float r = rcp_approx(x);
-    return fmaf(r, fmaf(-x, r, 1.0f), r);
-}
 
 // Layer constants of voxel_layer, from LayerRec in five 16-byte loads.
 struct LayerView {
     int spot_start, n_spots, energy_id;
-    float r80, A, B, C, rcut, lut_d0, lut_inv, lut_step, hs_log, hs_pole, hw_arg, hw_num, hw_den, hw_lin;
+    float r80, A, B, C, rcut, lut_d0, lut_inv, lut_step, hs_log, hs_pole, hw_arg, hw_num, hw_edge, hw_lin;
 };
 __device__ __forceinline__ LayerView load_layer(const LayerRec *L) {
     const float4 *v = reinterpret_cast<const float4 *>(L);
@@ -108,10 +104,16 @@ __device__ __forceinline__ LayerView load_layer(const LayerRec *L) {
 // nuclearHalo, IMPTClasses.cu:69-121).  `dw` = |voxel - source| - wet.  The
 // LUT row is computed where the depths are evenly spaced (lut_step > 0; the
 // interpolant is continuous, so a product rounded across a row boundary does
-// not matter) and searched for otherwise.  The logarithms and the quotients
-// that only shift sigma_h or the halo weight by a small term use the
-// approximate forms (2^-22, 1 ulp): at these terms' sizes their error stays
-// below 2e-8 of the halo weight and below the rounding of sigma_h.
+// not matter) and searched for otherwise.
+//
+// Errors against 64 bits over all energies and depths (rms, largest), in
+// brackets the same with logf, hypotf and IEEE divisions throughout: pf 6.3e-8,
+// 2.5e-7 (6.5e-8, 3.1e-7); hf relative to pf 4.3e-9, 6.5e-8 (5.7e-9, 7.3e-8);
+// ps2 4.6e-8, 1.5e-7 (the same); hs2 8.8e-8, 4.6e-7 (1.1e-7, 5.8e-7).  The
+// approximate logarithms and reciprocals serve only the small terms of sigma_h
+// and of the halo weight; pf and hf are quotients with their remainder added,
+// ps2 and hs2 take a Newton step.  IEEE forms throughout cost the batch kernel
+// 19 % (2.83 -> 3.37 ms).
 __device__ __forceinline__ VoxelLayer voxel_layer(const LayerView &L, const ProtonTables &t, int l, float wet, float dw) {
     const int n = t.lut_len;
     int i;
@@ -138,15 +140,20 @@ __device__ __forceinline__ VoxelLayer voxel_layer(const LayerView &L, const Prot
     const float hs = fmaf(w, fmaf(-7.4e-5f, w, 0.06f), fmaf(L.hs_log, log2_approx(w + 3.0f), 2.85f)) -
                      L.hs_pole * rcp_approx(sqr(w - r80 - 5.0f));
     const float hw = fmaf(0.052f * kLn2, log2_approx(fmaf(w, L.hw_arg, 1.13f)),
-                          fmaf(L.hw_num, rcp_approx(L.hw_den - sqr(w)), -L.hw_lin * w));
+                          fmaf(L.hw_num, rcp_approx((L.hw_edge - w) * (L.hw_edge + w)), -L.hw_lin * w));
     const float sigma_h = fmaxf(hs, 0.0f);
     const float wh = clampf(hw, 0.0f, 0.9f);
-    const float rt = recip(sqr(sigma_t)), rh = recip(fmaf(sigma_t, sigma_t, sqr(sigma_h)));
+    const float t2 = sqr(sigma_t), h2 = fmaf(sigma_t, sigma_t, sqr(sigma_h));
+    const float rt = rcp_approx(t2), rh = rcp_approx(h2);
+    auto over_2pi = [](float a, float s2, float r) {  // a / (2 pi s2), r ~ 1 / s2
+        const float inv = r * (0.5f / CUDART_PI_F), q = a * inv;
+        return fmaf(fmaf(-2.0f * CUDART_PI_F * s2, q, a), inv, q);
+    };
     VoxelLayer o;
-    o.pf = (1.0f - wh) * idd * (0.5f / CUDART_PI_F) * rt;
-    o.hf = wh * idd * (0.5f / CUDART_PI_F) * rh;
-    o.ps2 = (-0.5f * kLog2e) * rt;
-    o.hs2 = (-0.5f * kLog2e) * rh;
+    o.pf = over_2pi((1.0f - wh) * idd, t2, rt);
+    o.hf = over_2pi(wh * idd, h2, rh);
+    o.ps2 = (-0.5f * kLog2e) * fmaf(rt, fmaf(-t2, rt, 1.0f), rt);
+    o.hs2 = (-0.5f * kLog2e) * fmaf(rh, fmaf(-h2, rh, 1.0f), rh);
     return o;
 }
 

@@ -139,7 +139,7 @@ void build_proton_tables(const float *spots, int n_spots, const float *dvp, int 
         L.inv_vx = 1.0f / vsadx;
         L.inv_vy = 1.0f / vsady;
         L.lut_d0 = L.lut_inv = L.lut_step = 0.0f;
-        L.hs_log = L.hs_pole = L.hw_arg = L.hw_num = L.hw_den = L.hw_lin = 0.0f;
+        L.hs_log = L.hs_pole = L.hw_arg = L.hw_num = L.hw_edge = L.hw_lin = 0.0f;
         layers.push_back(L);
         s = t;
     }
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(128) layer_tables_kernel(Grid g, Frame f, Prot
     L.hs_pole = 0.22f * r80;
     L.hw_arg = 1.0f / (11.2f - 0.023f * r80);
     L.hw_num = 0.35f * ((0.0017f * sqr(r80)) - r80);
-    L.hw_den = sqr(r80 + 3.0f);
+    L.hw_edge = r80 + 3.0f;
     L.hw_lin = 1.61e-9f * sqr(r80 + 3.0f);
 }
 
