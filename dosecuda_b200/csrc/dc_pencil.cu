@@ -58,7 +58,11 @@ constexpr float kPrimaryBits = 26.0f;         // primary terms below 2^-26 of th
 // The spots a warp's pair loops read (broadcast), relative to the tile's
 // centre: U = p.x lx + p.y ly + p.z lz + p.w, W = q.x ly + q.y lz + q.z for
 // head-frame offsets l; per voxel step along z U changes by q.w and W by d.x,
-// d.y = (q.w^2 + d.x^2) / 4, and d.z = d.w = the spot's weight.  Spots with
+// d.y = (q.w^2 + d.x^2) / 4, and d.z = d.w = the spot's weight.  For listed
+// voxels, which share no centre, l is the position itself and p.w, q.z are the
+// spot's: U = p.x (lx - p.w) + p.y (ly - q.z) + p.z lz, W = q.x (ly - q.z) + q.y lz.
+// The differences are small and nearly exact where the Gaussian is not; sums
+// about a common origin would round at the size of lx.  Spots with
 // both terms fill the arrays from the front, those with the halo term alone
 // from the back.  One array per field keeps the lanes' stores free of bank
 // conflicts.
@@ -292,8 +296,9 @@ __device__ __forceinline__ void warp_beam(const ProtonTables &t, const PbExtra &
                             float r2[kVox];
 #pragma unroll
                             for (int v = 0; v < kVox; ++v) {
-                                const float U = fmaf(P.x, G.l[v].x, fmaf(P.y, G.l[v].y, fmaf(P.z, G.l[v].z, P.w)));
-                                const float W = fmaf(Q.x, G.l[v].y, fmaf(Q.y, G.l[v].z, Q.z));
+                                const float rx = G.l[v].x - P.w, ry = G.l[v].y - Q.z;
+                                const float U = fmaf(P.x, rx, fmaf(P.y, ry, P.z * G.l[v].z));
+                                const float W = fmaf(Q.x, ry, Q.y * G.l[v].z);
                                 r2[v] = fmaf(U, U, W * W);
                             }
                             r01 = make_float2(r2[0], r2[1]);
@@ -381,11 +386,12 @@ __device__ __forceinline__ void warp_beam(const ProtonTables &t, const PbExtra &
                     const float4 e = __ldg(t.axes + L.spot_start + s);
                     const float k2 = e.w * ty;
                     const float cu = fmaf(G.c.z, tx, G.c.x - a.x) + G.cl.x, cw = fmaf(G.c.z, ty, G.c.y - a.y) + G.cl.y;
+                    const float uw = kList ? a.x : fmaf(e.x, cu, e.y * cw), wz = kList ? a.y : e.w * cw;
                     const float du = fmaf(e.x, G.dz.x, fmaf(e.y, G.dz.y, e.z * G.dz.z)), dw = fmaf(e.w, G.dz.y, k2 * G.dz.z);
                     float mu = a.z;
                     if (!kAdj && x.mu != nullptr) mu = __ldg(x.mu + __float_as_int(a.w));
-                    mem.p[pos] = make_float4(e.x, e.y, e.z, fmaf(e.x, cu, e.y * cw));
-                    mem.q[pos] = make_float4(e.w, k2, e.w * cw, du);
+                    mem.p[pos] = make_float4(e.x, e.y, e.z, uw);
+                    mem.q[pos] = make_float4(e.w, k2, wz, du);
                     mem.d[pos] = make_float4(dw, 0.25f * fmaf(du, du, dw * dw), mu, mu);
                     if (kAdj) mem.orig[pos] = __float_as_int(a.w);
                 }
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(32 * kWarps, 6)
     WarpGeom<true> G;
     float gv[kVox], acc[kVox];
     const long long plane = (long long)g.nx * g.ny;
-    // Offsets are taken from the isocentre, not from a voxel of the warp: a
+    // Positions relative to the isocentre, not to a voxel of the warp: a
     // voxel's distances then do not depend on the list's other entries.
     G.c = make_float3(0.f, 0.f, 0.f);
     G.cl = make_float2(0.f, 0.f);

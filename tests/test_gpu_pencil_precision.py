@@ -62,3 +62,46 @@ def test_influence_on_the_axis():
         ref = _influence64(wet, float(r80[e]), float(sigma[e]), float(idd[e]), 0.0)
         sq += float(((dose / ref - 1.0) ** 2).mean())
     assert (sq / energies) ** 0.5 <= 6.55e-8
+
+
+def test_listed_voxels_far_from_the_isocentre():
+    """A listed voxel's distance from a spot 150 to 190 mm off the isocentre, at most 16 mm: in coordinates
+    relative to the spot three roundings and those of the unit vector, 4 x 2^-24 x 16 mm = 4e-6 mm, move
+    the Gaussian by r dr / sigma^2 = 16 x 4e-6 / 36 = 2e-6, the exponent's own rounding (5 x 2^-23) by
+    6e-7 and the parameters by 1e-6: 4e-6.  Coordinates relative to the isocentre would move it by
+    190 / 16 times the first figure, 2e-5."""
+    from dosecuda_b200 import engine
+    r80, sigma, idd = np.array([120.0], np.single), np.array([6.0], np.single), np.array([1.5], np.single)
+    model = _model(sigma, idd, r80)
+    shape = (12, 9, 16)  # exact coordinates: gantry 0, powers of two
+    sp = 2.0
+    rng = np.random.default_rng(3)
+    for sx, sy in ((160.0, -152.0), (-184.0, 176.0), (150.5, 188.25)):
+        grid = types.SimpleNamespace(spacing=np.array([sp] * 3), origin=np.array([0.0, 0.0, 0.0]))
+        # head x, y = -/+ image x, z at gantry 0: the volume lies around the spot's axis
+        for fx, fz in ((1, 1), (-1, 1), (1, -1), (-1, -1)):
+            iso = np.array([16.0 - fx * sx, 8.0, 12.0 - fz * sy], np.single)
+            beam = types.SimpleNamespace(iso=iso, gantry_angle=0.0, couch_angle=0.0,
+                                         spot_list=np.array([[sx, sy, 1.0, 0.0]], np.single))
+            wet = rng.uniform(0.5, 11.0, shape).astype(np.single)
+            w = torch.as_tensor(wet, device="cuda")
+            plan = engine.ProtonBeamPlan(grid, beam, model)
+            vox = torch.arange(wet.size, device="cuda", dtype=torch.int32)
+            dose = plan.dose_list(w, vox).cpu().numpy().reshape(shape)
+            k, j, i = np.meshgrid(*[np.arange(m, dtype=np.float64) * sp for m in shape], indexing="ij")
+            x, y, z = i - iso[0], j - iso[1], k - iso[2]
+            # the frame turns by 180 degrees, with the sine of the float32 pi
+            s180 = np.sin(np.float64(np.float32(np.pi)))
+            h = np.stack((x - y * s180, z, -x * s180 - y))
+            t = np.array([sx / float(model.VSADX), sy / float(model.VSADY), -1.0])
+            ray = h - np.array([sx, sy, 0.0])[:, None, None, None]
+            cross = np.cross(ray, t, axisa=0, axisc=0)
+            r2 = (cross ** 2).sum(0) / (t ** 2).sum()
+            near = r2 < 16.0 ** 2
+            if not near.any():
+                continue
+            ref = _influence64(wet, 120.0, 6.0, 1.5, r2)
+            assert np.abs(dose / ref - 1.0)[near].max() <= 4e-6
+            break
+        else:
+            raise AssertionError("the volume lies beside the spot")
