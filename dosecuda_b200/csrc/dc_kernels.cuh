@@ -77,7 +77,7 @@ struct __align__(16) LayerRec {
     float inv_vx, inv_vy;    // 1 / VSADX, 1 / VSADY
     float it2_min;           // smallest SpotRec::inv_t2 of the layer
     // device: first depth of the layer's LUT row, 1 / step and step (0 unless
-    // the depths are evenly spaced)
+    // the depths are evenly spaced, to the last bit)
     float lut_d0, lut_inv, lut_step;
     // device: coefficients of the nuclear halo's sigma (log and pole terms)
     // and weight (log argument, quotient, linear term) at this R80

@@ -106,9 +106,10 @@ __device__ __forceinline__ LayerView load_layer(const LayerRec *L) {
 
 // Per (voxel, layer) Gaussian parameters (interpolateProtonLUT, sigmaAir,
 // nuclearHalo, IMPTClasses.cu:69-121).  `dw` = |voxel - source| - wet.  The
-// LUT row is computed where the depths are evenly spaced (lut_step > 0; the
-// interpolant is continuous, so a product rounded across a row boundary does
-// not matter) and searched for otherwise.
+// LUT row is computed where the depths are evenly spaced (lut_step > 0: every
+// difference of neighbouring depths is the step, so the factor is the searched
+// form's; the interpolant is continuous, so a product rounded across a row
+// boundary does not matter) and searched for otherwise.
 //
 // Errors against 64 bits over all energies and depths (rms, largest), in
 // brackets the same with logf, hypotf and IEEE divisions throughout: pf 6.3e-8,
@@ -124,7 +125,9 @@ __device__ __forceinline__ VoxelLayer voxel_layer(const LayerView &L, const Prot
     float fac;
     if (L.lut_step > 0.0f) {
         i = min(max((int)ceilf((wet - L.lut_d0) * L.lut_inv), 0), n);
-        fac = (wet - fmaf((float)(i - 1), L.lut_step, L.lut_d0)) * L.lut_inv;
+        const float past = wet - fmaf((float)(i - 1), L.lut_step, L.lut_d0);
+        fac = past * L.lut_inv;
+        fac = fmaf(fmaf(-L.lut_step, fac, past), L.lut_inv, fac);  // past / step, rounded once
     } else {
         const float *D = t.lut_depths + (size_t)L.energy_id * n;
         int a = 0, b = n;

@@ -276,7 +276,10 @@ __global__ void __launch_bounds__(128) layer_tables_kernel(Grid g, Frame f, Prot
     const float *S = t.lut_sigmas + (size_t)L.energy_id * lut_len;
     const float step = lut_len > 1 ? (D[lut_len - 1] - D[0]) / (float)(lut_len - 1) : 0.0f;
     bool even = step > 0.0f;
-    for (int q = lane; q < lut_len; q += 32) even = even && D[q] == fmaf((float)q, step, D[0]);
+    // rows at d0 + q step with differences of exactly one step: a table in
+    // tenths of a mm has neither sum nor difference exact in binary
+    for (int q = lane; q < lut_len; q += 32)
+        even = even && D[q] == fmaf((float)q, step, D[0]) && (q == 0 || D[q] - D[q - 1] == step);
     even = __all_sync(0xffffffffu, even);
     // |sigma| over the rows up to the first one deeper than wmax (that row
     // included: it brackets wmax from above)

@@ -105,3 +105,24 @@ def test_listed_voxels_far_from_the_isocentre():
             break
         else:
             raise AssertionError("the volume lies beside the spot")
+
+
+@pytest.mark.parametrize("step", [0.7, 1.5])
+def test_depth_tables_in_decimal_steps(step):
+    """Depths q x 0.7 in float32 follow the even spacing bit for bit while their differences do not (up to
+    2.6e-5 of the step); a depth dose that goes up and down by a factor of 3 from row to row shows a factor
+    past / step instead of past / (difference).  The interpolation takes two roundings (2^-23), the pair's
+    influence 3e-7: 1e-6 in all.  Differences of 1.5 are exact."""
+    from dosecuda_b200 import engine
+    r80 = np.array([250.0], np.single)
+    model = _model([4.0], [1.0], r80)
+    model.lut_depths = model.lut_depths * np.float32(step)
+    model.lut_idds = np.where(np.arange(400) % 2 == 0, np.float32(1.0), np.float32(3.0))[None].astype(np.single)
+    grid = types.SimpleNamespace(spacing=np.array([2.0, 0.25, 2.0]), origin=np.array([0.0, -512.0, 0.0]))
+    beam = types.SimpleNamespace(iso=np.zeros(3, np.single), gantry_angle=0.0, couch_angle=0.0,
+                                 spot_list=np.array([[0.0, 0.0, 1.0, 0.0]], np.single))
+    wet = np.random.default_rng(5).uniform(0.05, 24.9, (1, 4096, 1)).astype(np.single)
+    dose = engine.proton_dose(torch.as_tensor(wet, device="cuda"), grid, beam, engine.ProtonModelDevice(model)).cpu().numpy()
+    mm = (wet * np.float32(10.0)).astype(np.float64)
+    idd = np.interp(mm, model.lut_depths[0].astype(np.float64), model.lut_idds[0].astype(np.float64))
+    assert np.abs(dose / _influence64(wet, 250.0, 4.0, idd, 0.0) - 1.0).max() <= 1e-6
