@@ -136,6 +136,13 @@ void build_proton_tables(const float *spots, int n_spots, const float *dvp, int 
             L.y1 = std::max(L.y1, spot_recs[q].y);
             L.it2_min = std::min(L.it2_min, spot_recs[q].inv_t2);
         }
+        // a spot without a finite position reaches every voxel (and makes its
+        // dose NaN): the range, which leaves NaN out, must not cull it
+        for (int q = s; q < t; ++q)
+            if (!std::isfinite(spot_recs[q].x) || !std::isfinite(spot_recs[q].y)) {
+                L.x0 = L.y0 = -INFINITY;
+                L.x1 = L.y1 = INFINITY;
+            }
         L.inv_vx = 1.0f / vsadx;
         L.inv_vy = 1.0f / vsady;
         L.lut_d0 = L.lut_inv = L.lut_step = 0.0f;

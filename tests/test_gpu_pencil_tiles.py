@@ -98,3 +98,17 @@ def test_batch_equals_the_one_beam_sum_in_every_variant():
     for v in range(b.n_variants):
         for d, p in zip(b.dose(variant=v), parts):
             assert np.abs(d.cpu().numpy() - p[4]).max() <= TOL * p[4].max()
+
+
+def test_spot_positions_that_are_not_finite():
+    """A spot at NaN or infinity makes the dose NaN in every voxel its layer reaches, however far the voxel's
+    tile is from the layer's other spots (here up to 370 mm)."""
+    from dosecuda_b200 import engine
+    model, grid, beam, wet, ref = _case((5, 9, 200), 3, 20, 30.0, 0.0, spread=8.0)
+    deep = 1.1 * float(model.divergence_params[int(beam.spot_list[0, 3]), 1])
+    for bad in (np.nan, np.inf):
+        spots = beam.spot_list.copy()
+        spots[0, 0] = bad
+        dose = engine.proton_dose(torch.as_tensor(wet, device="cuda"), grid, beam, engine.ProtonModelDevice(model),
+                                  spots=spots).cpu().numpy()
+        assert np.array_equal(np.isnan(dose), (wet * np.float32(10.0)) <= np.float32(deep))
