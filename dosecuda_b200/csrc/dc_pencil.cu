@@ -417,6 +417,13 @@ __device__ __forceinline__ void warp_beam(const ProtonTables &t, const PbExtra &
 // of six beams 3.24 -> 2.83 ms, 256 x 256 x 160 1.35 -> 1.27).
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 
+// WET of voxel u in mm.  At -infinity the air sigma is infinite and the dose 0:
+// no voxel.
+__device__ __forceinline__ float voxel_wet(const float *__restrict__ wet_s, long long u) {
+    const float w = __ldg(wet_s + u) * 10.0f;
+    return w == -INFINITY ? INFINITY : w;
+}
+
 // Geometry of the tile with low corner (i0, j0, k0) and, when a layer of the
 // beam comes near its box, the voxels' depths; false when none does.  gv: the
 // voxels' gradients where grad is given (0 outside the grid).
@@ -453,7 +460,7 @@ __device__ __forceinline__ bool tile_geom(const Grid &g, const Frame &f, const P
         if (!inside) continue;
         const long long u = (long long)i + (long long)g.nx * (j + (long long)g.ny * k);
         if (!DC_IN_BOUNDS(u, g.n(), 25)) continue;
-        G.wet[v] = __ldg(wet_s + u) * 10.0f;
+        G.wet[v] = voxel_wet(wet_s, u);
         G.dw[v] = distance_to_source(f, voxel_xyz(g, f, i, j, k)) - G.wet[v];
         if (grad != nullptr) gv[v] = __ldg(grad + u);
     }
@@ -539,7 +546,7 @@ __global__ void __launch_bounds__(32 * kWarps, 6)
         acc[v] = 0.0f;
         if (valid && DC_IN_BOUNDS(u, g.n(), 21)) {
             have = true;
-            G.wet[v] = __ldg(wet_s + u) * 10.0f;
+            G.wet[v] = voxel_wet(wet_s, u);
             G.dw[v] = distance_to_source(f, p) - G.wet[v];
             if (kAdj) gv[v] = __ldg(x.grad_dose + e);
             lo[0] = fminf(lo[0], G.l[v].x), hi[0] = fmaxf(hi[0], G.l[v].x);

@@ -112,3 +112,19 @@ def test_spot_positions_that_are_not_finite():
         dose = engine.proton_dose(torch.as_tensor(wet, device="cuda"), grid, beam, engine.ProtonModelDevice(model),
                                   spots=spots).cpu().numpy()
         assert np.array_equal(np.isnan(dose), (wet * np.float32(10.0)) <= np.float32(deep))
+
+
+def test_depth_of_minus_infinity():
+    """At WET -infinity the air sigma is infinite: the voxel's dose is 0, its neighbours' doses are as they are
+    without it."""
+    from dosecuda_b200 import engine
+    model, grid, beam, wet, ref = _case((9, 13, 40), 3, 20, 30.0, 0.0, spread=8.0)
+    wet[4, 6, 20] = -np.inf
+    plan = engine.ProtonBeamPlan(grid, beam, model)
+    every = torch.arange(wet.size, dtype=torch.int32)
+    for dose in (plan.dose(torch.as_tensor(wet, device="cuda")),
+                 plan.dose_list(torch.as_tensor(wet, device="cuda"), every).view(wet.shape)):
+        dose = dose.cpu().numpy()
+        assert dose[4, 6, 20] == 0.0
+        dose[4, 6, 20] = ref[4, 6, 20]
+        assert np.abs(dose - ref).max() <= TOL * ref.max()
