@@ -261,8 +261,10 @@ __device__ __forceinline__ void warp_beam(const ProtonTables &t, const PbExtra &
                 ratio = fmaxf(ratio, q == q ? q : INFINITY);  // no halo: the primary is never left out
                 dmin = fminf(dmin, pv[v].hs2 - pv[v].ps2);
             }
-            // smallest r^2 from which on every primary term is below 2^-26 of its halo term
-            const float rp = (kPrimaryBits + log2_approx(ratio)) * rcp_approx(dmin) * 1.0001f;
+            // smallest r^2 from which on every primary term is below 2^-26 of its halo term; a lane without a
+            // voxel has no say
+            const bool any = act[0] || act[1] || act[2] || act[3];
+            const float rp = any ? (kPrimaryBits + log2_approx(ratio)) * rcp_approx(dmin) * 1.0001f : 0.0f;
             // Lateral cut-off of this tile for this layer: 6 x the widest halo
             // sigma of its active voxels, never wider than the layer's bound.  A
             // spot whose axis stays farther than that from the tile's box lies

@@ -128,3 +128,28 @@ def test_depth_of_minus_infinity():
         assert dose[4, 6, 20] == 0.0
         dose[4, 6, 20] = ref[4, 6, 20]
         assert np.abs(dose - ref).max() <= TOL * ref.max()
+
+
+@pytest.mark.parametrize("shape", [(16, 24, 40), (15, 22, 37)])  # full tiles, and tiles with lanes without a voxel
+def test_halo_far_from_the_primary(shape):
+    """One spot in a smooth depth: most of the volume is reached by its halo alone, whose dose is compared
+    relative to itself, down to 1e-6 of the maximum.  There the exponent is at most 14: sigma_h to 4.6e-7 and the
+    product's rounding move it by 8e-6, positions to 1e-5 mm by 1e-5 r / sigma_h^2 = 3e-6, exp2 itself 2^-22."""
+    import oracle
+    from dosecuda_b200 import engine
+    model, grid, beam, _, _ = _case((1, 1, 1), 2, 1, 0.0, 0.0)
+    beam.spot_list[:, :2] = 4.0, -3.0
+    beam.spot_list[:, 3] = 60.0, 75.0
+    k, j, i = np.meshgrid(*[np.arange(n) for n in shape], indexing="ij")
+    wet = (3.0 + 0.2 * j + 0.01 * i - 0.02 * k).astype(np.single)
+    ref, _ = oracle.proton_dose(wet, grid.spacing, grid.origin, beam.iso, 0.0, 0.0, model, beam.spot_list)
+    w = torch.as_tensor(wet, device="cuda")
+    plan = engine.ProtonBeamPlan(grid, beam, model)
+    seen = ref > 1e-6 * ref.max()
+    assert 0.5 < seen.mean()
+    for dose in (plan.dose(w), plan.dose_list(w, torch.arange(wet.size, dtype=torch.int32)).view(shape)):
+        assert np.abs(dose.cpu().numpy() / ref - 1.0)[seen].max() <= 1.2e-5
+    mu = torch.as_tensor(beam.spot_list[:, 2].astype(np.float64), device="cuda")
+    far = (ref < 1e-3 * ref.max()) & seen  # the adjoint of a gradient on the halo's voxels only
+    got = float(plan.adjoint(w, torch.as_tensor(far.astype(np.single), device="cuda")) @ mu)
+    assert abs(got / ref[far].sum() - 1.0) <= 1.2e-5
