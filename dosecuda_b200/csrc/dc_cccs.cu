@@ -41,6 +41,7 @@
 // 0.076 -> 0.065; 143 x 131 x 97 at 3 mm, shaped field 1.66 -> 1.27; 36 x 32 x 30
 // at 4 mm 0.060 -> 0.039; 91 x 82 x 35 at 2.5 mm, 4 x 2 cm 0.080 -> 0.056.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <type_traits>
 
@@ -397,11 +398,24 @@ DC_BOUNDS_TAKE(take_bounds_cccs)
 
 namespace {
 
+// Most bytes of a staged box: two blocks per SM.
+constexpr size_t kMostBytes = 104 * 1024;
+
+// Opts the kernel in to kMostBytes of dynamic shared memory, once per device
+// and to the same limit whatever the launch needs: the limit belongs to the
+// function, and calls of several threads share it.
+template <class K>
+void allow_shared(K *kernel, size_t smem, int device, std::atomic<bool> (&done)[64]) {
+    if (smem <= 40 * 1024) return;  // the static arrays count too
+    if (device < 64 && done[device].load(std::memory_order_acquire)) return;
+    DC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostBytes));
+    if (device < 64) done[device].store(true, std::memory_order_release);
+}
+
 // Fills B for a tile and returns the staged box's bytes.  Where no near sample
 // fits (spacings far below the cones' ray lengths never do that; very uneven
 // ones may) only the tile's own texels are staged and all others are fetched.
 size_t cccs_plan(const CccsCones &C, const Grid &g, CccsPlan &B) {
-    constexpr size_t kMostBytes = 104 * 1024;  // two blocks per SM
     int total = 0, longest = 0;
     for (int c = 0; c < C.n_cones; ++c) {
         B.n_zero[c] = C.n_steps[c] > 0 && C.rl10[C.step_off[c] + C.n_steps[c] - 1] == 0.0f;
@@ -440,8 +454,8 @@ void enqueue_cccs(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsC
     KernelTimer kt(ctx, "cccs", s);
     CccsPlan B;
     const size_t smem = cccs_plan(C, g, B);
-    if (smem > 40 * 1024)  // the static arrays count too
-        DC_CUDA(cudaFuncSetAttribute(cccs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<bool> allowed[64] = {};
+    allow_shared(cccs_kernel, smem, ctx.device, allowed);
     const dim3 grid((unsigned)((g.nx + Tile::x - 1) / Tile::x), (unsigned)((g.ny + Tile::y - 1) / Tile::y),
                     (unsigned)((g.nz + Tile::z - 1) / Tile::z));
     cccs_kernel<<<grid, kThreads, smem, s>>>(g, f, C, B, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex, w.electron, w.mask,
@@ -462,8 +476,8 @@ void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, cons
     const size_t box = (size_t)B.wx * B.wy * (B.wz - 1) * sizeof(float4);
     const int per_block = (int)std::min<size_t>(kListVoxels, std::max<size_t>(1, 56 * 1024 / box));
     const size_t smem = box * per_block;
-    if (smem > 40 * 1024)
-        DC_CUDA(cudaFuncSetAttribute(cccs_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<bool> allowed[64] = {};
+    allow_shared(cccs_list_kernel, smem, ctx.device, allowed);
     cccs_list_kernel<<<(unsigned)((n + per_block - 1) / per_block), kListThreads, smem, s>>>(
         g, f, C, B, per_block, reach * 1.0001f, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex, w.electron, w.mask, voxels,
         n, out);

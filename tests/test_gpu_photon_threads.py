@@ -1,0 +1,61 @@
+"""Photon beams (dc_photon_beam.cu) used from several threads and on several streams at once."""
+import threading
+import types
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _beam(engine, model, shape, spacing, half_x, half_y=25.0, gantry=20.0):
+    import torch
+
+    from dosecuda_b200.plan_imrt import IMRTControlPoint
+    nz, ny, nx = shape
+    grid = types.SimpleNamespace(spacing=np.array([spacing] * 3),
+                                 origin=np.array([-n * spacing / 2 for n in (nx, ny, nz)]))
+    x12 = np.where(np.abs(model.mlc_offsets) <= half_y, half_x, 0.0)
+    mlc = np.array(np.vstack((-x12, x12, model.mlc_offsets, model.mlc_widths)), dtype=np.single).T
+    cp = IMRTControlPoint(np.zeros(3, np.single), 100.0, mlc, gantry, 0.0, 0.0, None, None)
+    beam = engine.PhotonBeam(grid, shape)
+    beam.set_density(torch.ones(shape, device="cuda"))
+    return beam, cp
+
+
+def test_doses_of_several_spacings_from_several_threads():
+    """The CCCS of a fine grid opts in to more shared memory than that of a coarser one; either may run between
+    the other's opt-in and its launch.  Every call has to be accepted and give the dose it gives alone."""
+    import torch
+
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTPlan
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    beams, want, outs = [], [], []
+    for spacing in (1.0, 1.5, 1.25):
+        beam, cp = _beam(engine, model, (8, 12, 16), spacing, 25.0)
+        beam.terma(model, cp)
+        beams.append(beam)
+        want.append((beam.dose(), beam.probe()))
+        outs.append((torch.empty_like(want[-1][0]), torch.empty_like(want[-1][1])))
+    streams = [torch.cuda.Stream() for _ in beams]
+    torch.cuda.synchronize()
+    failed = []
+
+    def work(q):
+        try:
+            for _ in range(400):
+                beams[q].dose(out=outs[q][0], stream=streams[q])
+                beams[q].probe(out=outs[q][1], stream=streams[q])
+        except Exception as e:  # a launch that was refused
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(q,)) for q in range(len(beams))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed[0]
+    for (dose, probe), (d, p) in zip(want, outs):
+        assert torch.equal(dose, d) and torch.equal(probe, p)
