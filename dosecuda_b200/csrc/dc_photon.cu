@@ -258,9 +258,11 @@ __global__ void __launch_bounds__(128) terma_kernel(Grid g, Frame f, PhotonParam
 
     const bool act = !(T <= 0.01f);
     if (!act && dose && v_ok) dose[v] = 0.0f;
-    const unsigned live = __activemask();
-    const unsigned bal = __ballot_sync(live, act);
-    if (threadIdx.x == 0) mask[((long long)k * g.ny + j) * gridDim.x + blockIdx.x] = bal;  // a warp is a row's 32 voxels
+    // a warp is 32 voxels of a row, the last one of each row those that are left; the ballot waits for all of
+    // them, wherever they are in the code above
+    const int left = g.nx - (int)(blockIdx.x * 32);
+    const unsigned bal = __ballot_sync(left >= 32 ? 0xffffffffu : (1u << left) - 1u, act);
+    if (threadIdx.x == 0) mask[((long long)k * g.ny + j) * gridDim.x + blockIdx.x] = bal;
     if (act) {
         const int lane = threadIdx.x & 31;
         const int leader = __ffs(bal) - 1;
