@@ -316,8 +316,8 @@ constexpr int kListThreads = 288, kListVoxels = 4;
 __global__ void __launch_bounds__(kListThreads, 5)
     cccs_list_kernel(Grid g, Frame f, const __grid_constant__ CccsCones C, const __grid_constant__ CccsPlan B,
                      int per_block, float reach, float sp_cm, float dose_scale, const float4 *__restrict__ dirs,
-                     cudaTextureObject_t td_tex, const float *__restrict__ electron, const unsigned *__restrict__ mask,
-                     const int *__restrict__ voxels, int n, float *__restrict__ out) {
+                     cudaTextureObject_t td_tex, const float *__restrict__ electron, const int *__restrict__ voxels,
+                     int n, float *__restrict__ out) {
     extern __shared__ float4 s_boxes[];  // [per_block][wz - 1][wy][wx]
     __shared__ float4 s_dir[kMaxCones * 12];
     __shared__ float s_rl10[kMaxConeSteps];
@@ -331,9 +331,9 @@ __global__ void __launch_bounds__(kListThreads, 5)
         if (e0 + tid < n) v = __ldg(voxels + e0 + tid);
         if (v < 0 || (long long)v >= g.n()) v = -1;
         if (v >= 0) {
-            const int row = v / g.nx, i = v - row * g.nx;
-            const long long word = (long long)row * mask_words(g.nx) + (i >> 5);
-            if (!(__ldg(mask + word) >> (i & 31) & 1u)) v = -1;
+            // masked by the texel itself (read at its centre), which a fluence map may have scaled since the mask
+            const int row = v / g.nx, i = v - row * g.nx, k = row / g.ny, j = row - k * g.ny;
+            if (tex3D<float2>(td_tex, i + 0.5f, j + 0.5f, k + 0.5f).x <= 0.01f) v = -1;
         }
         s_voxel[tid] = v;
         if (v >= 0) {
@@ -479,8 +479,8 @@ void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, cons
     static std::atomic<bool> allowed[64] = {};
     allow_shared(cccs_list_kernel, smem, ctx.device, allowed);
     cccs_list_kernel<<<(unsigned)((n + per_block - 1) / per_block), kListThreads, smem, s>>>(
-        g, f, C, B, per_block, reach * 1.0001f, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex, w.electron, w.mask, voxels,
-        n, out);
+        g, f, C, B, per_block, reach * 1.0001f, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex, w.electron, voxels, n,
+        out);
     check_launch("cccs_list_kernel");
 }
 

@@ -35,3 +35,29 @@ def test_dose_and_adjoint_agree(shape):
         g = torch.randn(shape, generator=gen).cuda()
         lhs, rhs = float((g.double() * dose).sum()), float((fb.adjoint(g).reshape(F.shape) * F.double()).sum())
         assert abs(lhs - rhs) <= 2e-3 * float((g.double().abs() * dose).sum())
+
+
+def test_probe_after_a_fluence_dose():
+    """The probe leaves out voxels by their TERMA as it is in the beam: where the map is 0 it gives 0, although the
+    dose there, masked by the unmodulated TERMA, holds scatter from the open half.  Elsewhere both agree."""
+    import torch
+
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTControlPoint, IMRTPlan
+
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    shape, sp = (24, 20, 28), 3.0
+    nz, ny, nx = shape
+    grid = types.SimpleNamespace(spacing=np.array([sp] * 3), origin=np.array([-n * sp / 2 for n in (nx, ny, nz)]))
+    x12 = np.where(np.abs(model.mlc_offsets) <= 30.0, 30.0, 0.0)
+    mlc = np.array(np.vstack((-x12, x12, model.mlc_offsets, model.mlc_widths)), dtype=np.single).T
+    cp = IMRTControlPoint(np.zeros(3, np.single), 100.0, mlc, 0.0, 0.0, 0.0, None, None)
+    fb = engine.PhotonFluenceBeam.field_map(torch.ones(shape, device="cuda"), grid, model, cp, pitch=5.0)
+    F = torch.ones((fb.nb, fb.na), device="cuda")
+    F[:, : fb.na // 2] = 0.0
+    dose = fb.dose(F).reshape(-1)
+    probe = fb.beam.probe(torch.arange(dose.numel(), device="cuda", dtype=torch.int32))
+    kept = probe != 0
+    assert torch.equal(probe[kept], dose[kept])
+    left_out = (dose > 1e-3 * dose.max()) & ~kept  # scatter under the closed half
+    assert 20 <= int(left_out.sum()) < int(kept.sum())
