@@ -20,6 +20,7 @@
 #include <cstring>
 #include <iterator>
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "../../include/dosecuda.h"
@@ -363,15 +364,23 @@ int dc_photon_beam_terma(dc_photon_beam *b, const dc_photon_model *model, const 
         DC_CUDA(cudaSetDevice(b->device));
         DeviceContext &ctx = context(b->device);
         float *t0 = static_cast<float *>(b->terma0.ensure((size_t)b->g.n() * sizeof(float)));
-        enqueue_terma(ctx, b->g, b->f, b->P, b->C, b->work(), nullptr, t0, as_stream(stream));
+        const PhotonWork w = b->work();
+        cudaStream_t s = as_stream(stream);
+        {
+            // the head factors, the side stream and its events are the
+            // context's: TERMA passes of several beams take turns
+            std::lock_guard<std::mutex> lk(ctx.mu);
+            ctx.begin_call(s);
+            enqueue_terma(ctx, b->g, b->f, b->P, b->C, w, nullptr, t0, s);
+            ctx.end_call(s);
+        }
         if (terma_out_dev)
-            DC_CUDA(cudaMemcpyAsync(terma_out_dev, t0, (size_t)b->g.n() * sizeof(float), cudaMemcpyDeviceToDevice,
-                                    as_stream(stream)));
+            DC_CUDA(cudaMemcpyAsync(terma_out_dev, t0, (size_t)b->g.n() * sizeof(float), cudaMemcpyDeviceToDevice, s));
         b->have_terma = true;
         b->have_e0 = false;
         // the probe of this control point, selected on the host while the
         // TERMA kernels run
-        select_and_upload_probe(*b, as_stream(stream));
+        select_and_upload_probe(*b, s);
     });
 }
 

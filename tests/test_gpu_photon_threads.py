@@ -59,3 +59,43 @@ def test_doses_of_several_spacings_from_several_threads():
     assert not failed, failed[0]
     for (dose, probe), (d, p) in zip(want, outs):
         assert torch.equal(dose, d) and torch.equal(probe, p)
+
+
+def test_termas_of_two_beams_on_two_streams():
+    """Two beams' TERMA passes, enqueued on two streams without waiting and from two threads, share the
+    context's head factors: each has to be what it is alone.  A photon dose call uses the same buffer."""
+    import torch
+
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTPlan
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    pairs = [_beam(engine, model, (48, 56, 64), 3.0, hx, hy, ga) for hx, hy, ga in ((60.0, 50.0, 0.0), (15.0, 30.0, 75.0))]
+    want = [b.terma(model, cp, out=True).clone() for b, cp in pairs]
+    torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    streams = [torch.cuda.Stream() for _ in pairs]
+    for _ in range(10):
+        got = []
+        for (b, cp), s in zip(pairs, streams):
+            with torch.cuda.stream(s):
+                got.append(b.terma(model, cp, out=True, stream=s))
+        torch.cuda.synchronize()
+        for g, w in zip(got, want):
+            assert torch.equal(g, w)
+    bad = []
+
+    def work(q):
+        (b, cp), s = pairs[q], streams[q]
+        with torch.cuda.stream(s):
+            for _ in range(20):
+                g = b.terma(model, cp, out=True, stream=s)
+                s.synchronize()
+                if not torch.equal(g, want[q]):
+                    bad.append(q)
+
+    threads = [threading.Thread(target=work, args=(q,)) for q in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
