@@ -222,8 +222,10 @@ __global__ void __launch_bounds__(128) cccs_adjoint_kernel(Grid g, Frame f, Cccs
                     if (i0 < -1 || i0 >= g.nx || j0 < -1 || j0 >= g.ny) continue;
                     const long long cell = ((i0 + 1) >> 1) + (long long)Q.qx * ((j0 + 1) >> 1);
                     float *rec = quads + ((i0 + 1) & 1) * Q.part + ((j0 + 1) & 1) * 2 * Q.part + 4 * cell;
-                    const float wy1 = wT * wb, wy0 = wT - wy1;
-                    const float4 w4 = make_float4(wy0 - wy0 * wa, wy0 * wa, wy1 - wy1 * wa, wy1 * wa);
+                    // the weights' products are exact (multiples of 2^-24), so that each texel's part is rounded
+                    // once; a texel without weight takes nothing, whatever wT is
+                    const float a0 = 1.0f - wa, b0 = 1.0f - wb;
+                    const float4 w4 = make_float4(a0 * b0, wa * b0, a0 * wb, wa * wb);
                     const long long plane4 = 4LL * Q.qx * Q.qy;
 #pragma unroll
                     for (int dk = 0; dk < 2; ++dk) {
@@ -231,8 +233,9 @@ __global__ void __launch_bounds__(128) cccs_adjoint_kernel(Grid g, Frame f, Cccs
                         const float wz = dk ? wc : 1.0f - wc;
                         if ((unsigned)kk >= (unsigned)g.nz || wz == 0.0f) continue;
                         float *t = rec + plane4 * kk;
+                        auto part = [&](float w) { return w * wz != 0.0f ? wT * (w * wz) : 0.0f; };
                         if (DC_IN_BOUNDS(t - quads, 4 * Q.part - 3, 54))
-                            red_add4(t, make_float4(w4.x * wz, w4.y * wz, w4.z * wz, w4.w * wz));
+                            red_add4(t, make_float4(part(w4.x), part(w4.y), part(w4.z), part(w4.w)));
                     }
                 }
             }

@@ -61,3 +61,29 @@ def test_probe_after_a_fluence_dose():
     assert torch.equal(probe[kept], dose[kept])
     left_out = (dose > 1e-3 * dose.max()) & ~kept  # scatter under the closed half
     assert 20 <= int(left_out.sum()) < int(kept.sum())
+
+
+def test_adjoint_of_an_infinite_gradient():
+    """An infinite gradient at one voxel makes the beamlets infinite that its dose depends on, and none NaN: texels
+    with weight 0 take no part of it, and no part of a sample is a difference of infinities.  The voxel lies at
+    the surface, where TERMA and the electron term of all texels in reach are above 0."""
+    import torch
+
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTControlPoint, IMRTPlan
+
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    shape, sp = (9, 6, 10), 4.0
+    nz, ny, nx = shape
+    grid = types.SimpleNamespace(spacing=np.array([sp] * 3), origin=np.array([-n * sp / 2 for n in (nx, ny, nz)]))
+    x12 = np.where(np.abs(model.mlc_offsets) <= 100.0, 90.0, 0.0)
+    mlc = np.array(np.vstack((-x12, x12, model.mlc_offsets, model.mlc_widths)), dtype=np.single).T
+    cp = IMRTControlPoint(np.zeros(3, np.single), 100.0, mlc, 0.0, 0.0, 0.0, None, None)
+    fb = engine.PhotonFluenceBeam.field_map(torch.ones(shape, device="cuda"), grid, model, cp, pitch=5.0)
+    for at in ((4, 0, 5), (0, 2, 0), (8, 3, 9)):
+        g = torch.zeros(shape, device="cuda")
+        g[at] = 1.0
+        want = fb.adjoint(g) != 0
+        g[at] = float("inf")
+        got = fb.adjoint(g)
+        assert torch.equal(got == float("inf"), want) and bool((got[~want] == 0).all())
