@@ -31,15 +31,18 @@
 //    groups of threads, added in a fixed order: a masked tile has few voxels,
 //    and a narrow field few tiles.  Tiles of 8 x 8 x 4 without groups take 2 %
 //    less on 128^3 with a 10 x 10 cm field and 10 % less on a field that fills
-//    143 x 131 x 97 (14.7 staged texels per voxel instead of 38), but twice the
+//    143 x 131 x 97 at 3 mm (5.9 staged texels per voxel instead of 12.8), but twice the
 //    time under narrow fields; 8 x 4 x 4 with two groups lie between (3 and 5 %
 //    less, 1.4 times).  Which is better depends on the number of active voxels,
 //    which is on the device; launching both, one to return at once, costs 20 us.
 //
 // Measured (ms; before = all samples from the texture unit, one thread per
 // listed voxel): 128^3 at 2.5 mm, 10 x 10 cm field 0.889 -> 0.720, 2 x 2 cm field
-// 0.076 -> 0.065; 143 x 131 x 97 at 3 mm, shaped field 1.66 -> 1.27; 36 x 32 x 30
-// at 4 mm 0.060 -> 0.039; 91 x 82 x 35 at 2.5 mm, 4 x 2 cm 0.080 -> 0.056.
+// 0.076 -> 0.061; 143 x 131 x 97 at 3 mm, shaped field 1.66 -> 1.27; 36 x 32 x 30
+// at 4 mm 0.060 -> 0.039; 91 x 82 x 35 at 2.5 mm, 4 x 2 cm 0.080 -> 0.056; 10 x 10 cm
+// on 87^3 at 1.5 mm 1.45 -> 1.13, on 96^3 at 1 mm 2.65 -> 2.30 (there a tile stages 3705
+// texels; one voxel more of margin, 5355, made it 2.65, and a 2 cm field 0.28
+// instead of 0.24).
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -306,12 +309,12 @@ __global__ void __launch_bounds__(kThreads, 4)
 // field), bit for bit cccs_kernel's: the same samples from the same sources,
 // added in the order of its groups.  Tiles around so few voxels would stage far
 // more texels than they use, so each voxel has a box of its own, of which only
-// the texels within reach of its near samples are staged (some 250 at 128^3,
+// the texels within reach of its near samples are staged (some 150 at 128^3,
 // 2.5 mm), and the directions of a block's voxels are dealt to its threads.  A
 // block takes 4 voxels: 8 leave 27 warps per SM, 2 or half-masked blocks idle
 // threads.  Measured (us; before = one thread per listed voxel, every sample
-// from the texture unit), 34 k voxels of 128^3 at 2.5 mm: 2 cm field 69 -> 25, 10 cm
-// 76 -> 70, 20 cm 107 -> 132; 5 k of 64^3 at 3 mm 74 -> 21.
+// from the texture unit), 34 k voxels of 128^3 at 2.5 mm: 2 cm field 69 -> 24, 10 cm
+// 75 -> 60, 20 cm 108 -> 110; 5 k of 64^3 at 3 mm 74 -> 21.
 constexpr int kListThreads = 288, kListVoxels = 4;
 __global__ void __launch_bounds__(kListThreads, 5)
     cccs_list_kernel(Grid g, Frame f, const __grid_constant__ CccsCones C, const __grid_constant__ CccsPlan B,
@@ -430,7 +433,9 @@ size_t cccs_plan(const CccsCones &C, const Grid &g, CccsPlan &B) {
             B.n_far[c] = n - B.n_near[c];
             if (B.n_near[c] > 0) reach = std::max(reach, C.rl10[C.step_off[c] + B.n_far[c]]);
         }
-        auto halo = [&](float sp) { return (int)std::min(200.0, std::ceil((double)reach / sp * 1.0001)); };
+        // a sample's offset is rounded to 1/256 voxel, so up to 1/512 voxel past a whole number it still lies in
+        // that voxel, with no weight on the next; 1/600 leaves 3e-4 for the rounding of directions and products
+        auto halo = [&](float sp) { return (int)std::min(200.0, std::ceil((double)reach / sp - 1.0 / 600.0)); };
         B.hx = halo(g.sx), B.hy = halo(g.sy), B.hz = halo(g.sz);
         B.wx = Tile::x + 2 * B.hx + 1, B.wy = Tile::y + 2 * B.hy + 1, B.wz = Tile::z + 2 * B.hz + 1;
         return (size_t)B.wx * B.wy * (B.wz - 1) * sizeof(float4);
