@@ -21,7 +21,7 @@
 //  * A sample's coordinates are one fused multiply-add per axis: in voxels
 //    for the texture unit; in 1/256 voxel, rounded by adding 1.5 * 2^23, for
 //    shared memory, where the low byte is the fraction and the next the cell.
-//    The weights are the texture unit's own (box_sample): with plain products
+//    The weights are the texture unit's own (CornerWeights): with plain products
 //    of the fractions the dose would differ by 5e-5.
 //  * The tile's voxels above the TERMA mask (a bit per voxel, from the TERMA
 //    kernel) are compacted over the block's threads.
@@ -85,39 +85,64 @@ struct Tile {
 };
 static_assert(Tile::voxels * Tile::groups == kThreads, "a thread per voxel and group");
 
-// 256 x the trilinear (TERMA, density) at box coordinates tx, ty, tz (magic
-// floats in 1/256 voxel), with the texture unit's weights: the eight weights
-// are multiples of 1/256 that sum to 1, split off 1 by z, then x, then y, each
-// split rounded to 1/256, ties to the upper side except in the y split of the
-// lower x side (found by sampling volumes with a single non-zero texel at
-// 20000 fractions; every one of the 160000 weights agrees).  A register holds
-// the two z sides of a weight in 16-bit fields, so that one multiply-add
-// splits both and one byte permute shifts both; as floats they ride in the
-// paired lanes, like the texels in the box's records.  The index is kept
+// The texture unit's weights of a sample at box coordinates tx, ty, tz (magic
+// floats in 1/256 voxel): multiples of 1/256 that sum to 1, split off 1 by z,
+// then x, then y, each split rounded to 1/256, ties to the upper side except in
+// the y split of the lower x side (found by sampling volumes with a single
+// non-zero texel at 20000 fractions; every one of the 160000 weights agrees).
+// Times 256, both z sides of a weight in one pair.  A register holds the two in
+// 16-bit fields, so that one multiply-add splits both and one byte permute
+// shifts both; as floats they ride in the paired lanes.
+struct CornerWeights {
+    float2 u00, u10, u01, u11;  // of (x, y) corner (0, 0), (1, 0), (0, 1), (1, 1): lower z, upper z
+    __device__ __forceinline__ CornerWeights(float tx, float ty, float tz) {
+        const unsigned fx = __byte_perm(__float_as_uint(tx), 0, 0x4440), fy = __byte_perm(__float_as_uint(ty), 0, 0x4440);
+        const unsigned fz = __byte_perm(__float_as_uint(tz), 0, 0x4440);
+        const unsigned z = fz * 65535u + 256u;  // (256 - fz, fz)
+        const unsigned x1 = __byte_perm(z * fx + 0x00800080u, 0, 0x4341), x0 = z - x1;
+        const unsigned w11 = __byte_perm(x1 * fy + 0x00800080u, 0, 0x4341), w10 = x1 - w11;
+        const unsigned w01 = __byte_perm(x0 * fy + 0x007F007Fu, 0, 0x4341), w00 = x0 - w01;
+        auto pair = [](unsigned w) {  // both fields as floats: the mantissa of 2^23 + w
+            return __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7410)),
+                                          __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7432))),
+                              make_float2(-8388608.0f, -8388608.0f));
+        };
+        u00 = pair(w00), u10 = pair(w10), u01 = pair(w01), u11 = pair(w11);
+    }
+};
+__device__ __forceinline__ int box_cell(float t) { return __byte_perm(__float_as_uint(t), 0, 0x4441); }
+
+// 256 x the trilinear (TERMA, density) in a box of records.  The index is kept
 // inside the box whatever the coordinates.
-__device__ __forceinline__ float2 box_sample(const float4 *__restrict__ box, int row, int plane, int cap, float tx,
-                                             float ty, float tz) {
-    const unsigned bx = __float_as_uint(tx), by = __float_as_uint(ty), bz = __float_as_uint(tz);
-    const int cx = __byte_perm(bx, 0, 0x4441), cy = __byte_perm(by, 0, 0x4441), cz = __byte_perm(bz, 0, 0x4441);
-    const unsigned fx = __byte_perm(bx, 0, 0x4440), fy = __byte_perm(by, 0, 0x4440), fz = __byte_perm(bz, 0, 0x4440);
-    const float4 *p = box + min(cx + cy * row + cz * plane, cap);
-    const float4 a = p[0], b = p[1], c = p[row], d = p[row + 1];
-    const unsigned z = fz * 65535u + 256u;  // (256 - fz, fz)
-    const unsigned x1 = __byte_perm(z * fx + 0x00800080u, 0, 0x4341), x0 = z - x1;
-    const unsigned w11 = __byte_perm(x1 * fy + 0x00800080u, 0, 0x4341), w10 = x1 - w11;
-    const unsigned w01 = __byte_perm(x0 * fy + 0x007F007Fu, 0, 0x4341), w00 = x0 - w01;
-    auto pair = [](unsigned w) {  // both fields as floats: the mantissa of 2^23 + w
-        return __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7410)),
-                                      __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7432))),
-                          make_float2(-8388608.0f, -8388608.0f));
-    };
-    const float2 u00 = pair(w00), u10 = pair(w10), u01 = pair(w01), u11 = pair(w11);
-    const float2 t = __ffma2_rn(u11, make_float2(d.x, d.y), __ffma2_rn(u01, make_float2(c.x, c.y),
-                     __ffma2_rn(u10, make_float2(b.x, b.y), __fmul2_rn(u00, make_float2(a.x, a.y)))));
-    const float2 r = __ffma2_rn(u11, make_float2(d.z, d.w), __ffma2_rn(u01, make_float2(c.z, c.w),
-                     __ffma2_rn(u10, make_float2(b.z, b.w), __fmul2_rn(u00, make_float2(a.z, a.w)))));
-    return make_float2(t.x + t.y, r.x + r.y);
-}
+struct RecordBox {
+    const float4 *box;
+    int row, plane, cap;
+    __device__ __forceinline__ float2 operator()(float tx, float ty, float tz) const {
+        const float4 *p = box + min(box_cell(tx) + box_cell(ty) * row + box_cell(tz) * plane, cap);
+        const float4 a = p[0], b = p[1], c = p[row], d = p[row + 1];
+        const CornerWeights w(tx, ty, tz);
+        const float2 t = __ffma2_rn(w.u11, make_float2(d.x, d.y), __ffma2_rn(w.u01, make_float2(c.x, c.y),
+                         __ffma2_rn(w.u10, make_float2(b.x, b.y), __fmul2_rn(w.u00, make_float2(a.x, a.y)))));
+        const float2 r = __ffma2_rn(w.u11, make_float2(d.z, d.w), __ffma2_rn(w.u01, make_float2(c.z, c.w),
+                         __ffma2_rn(w.u10, make_float2(b.z, b.w), __fmul2_rn(w.u00, make_float2(a.z, a.w)))));
+        return make_float2(t.x + t.y, r.x + r.y);
+    }
+};
+// The same products and sums in a box of single texels, half the size.
+struct TexelBox {
+    const float2 *box;
+    int row, plane, cap;
+    __device__ __forceinline__ float2 operator()(float tx, float ty, float tz) const {
+        const float2 *p = box + min(box_cell(tx) + box_cell(ty) * row + box_cell(tz) * plane, cap);
+        const CornerWeights w(tx, ty, tz);
+        auto side = [&](const float2 *q, float w00, float w10, float w01, float w11) {
+            return __ffma2_rn(make_float2(w11, w11), q[row + 1], __ffma2_rn(make_float2(w01, w01), q[row],
+                   __ffma2_rn(make_float2(w10, w10), q[1], __fmul2_rn(make_float2(w00, w00), q[0]))));
+        };
+        const float2 l = side(p, w.u00.x, w.u10.x, w.u01.x, w.u11.x), h = side(p + plane, w.u00.y, w.u10.y, w.u01.y, w.u11.y);
+        return make_float2(l.x + h.x, l.y + h.y);
+    }
+};
 
 // One step of the recursions R = R e + T (1 - e), S = S (1 - b rho) + T rho
 // (the reference's Rp and Rs over their constant factors), e = exp(-a rho).
@@ -158,9 +183,10 @@ struct CccsVoxel {
 
 // am Rp + bm Rs of one direction r of cone c, from the farthest sample to the
 // voxel's own; b: the voxel's box coordinates (magic floats in 1/256 voxel).
+template <class Box>
 __device__ __forceinline__ float cccs_direction(const CccsCones &C, const CccsPlan &B, int c, const float *rl, float3 r,
                                                 float3 tc, float3 b, float sp_cm, cudaTextureObject_t td_tex,
-                                                const float4 *box, int row, int plane, int cap, float2 td0) {
+                                                const Box &box, float2 td0) {
     const float nal = -C.am[c] * kLog2e * sp_cm, nb = -C.bm[c] * sp_cm;
     const int n_far = B.n_far[c], n_near = B.n_near[c];
     float R = 0.0f, S = 0.0f;
@@ -191,7 +217,7 @@ __device__ __forceinline__ float cccs_direction(const CccsCones &C, const CccsPl
     r.z *= 256.0f;
     auto near_step = [&](int q) {
         const float L = rl[n_far + q];
-        float2 td = box_sample(box, row, plane, cap, fmaf(r.x, L, b.x), fmaf(r.y, L, b.y), fmaf(r.z, L, b.z));
+        float2 td = box(fmaf(r.x, L, b.x), fmaf(r.y, L, b.y), fmaf(r.z, L, b.z));
         td.x *= 1.0f / 256.0f;
         td.y *= 1.0f / 256.0f;
         cccs_step(td, nal, nb, R, S);
@@ -283,14 +309,14 @@ __global__ void __launch_bounds__(kThreads, 4)
         const CccsVoxel V(g, f, i, j, k);
         const float3 b = make_float3((float)((li + B.hx) * 256) + kMagic, (float)((lj + B.hy) * 256) + kMagic,
                                      (float)((lk + B.hz) * 256) + kMagic);
-        const int cap = (B.wz - 2) * plane + (B.wy - 2) * B.wx + B.wx - 2;
+        const RecordBox box{s_box, B.wx, plane, (B.wz - 2) * plane + (B.wy - 2) * B.wx + B.wx - 2};
         const float4 own = s_box[(lk + B.hz) * plane + (lj + B.hy) * B.wx + li + B.hx];
         for (int c = 0; c < C.n_cones; ++c) {
             float cone = 0.0f;
             for (int az = group; az < 12; az += Tile::groups) {
                 const float4 dv = s_dir[c * 12 + az];
                 const float x = cccs_direction(C, B, c, s_rl10 + C.step_off[c], V.tilt(g, dv), V.tc, b, sp_cm, td_tex,
-                                               s_box, B.wx, plane, cap, make_float2(own.x, own.z));
+                                               box, make_float2(own.x, own.z));
                 cone = fmaf(dv.w, x, cone);
             }
             sum += cone;
@@ -351,7 +377,7 @@ __global__ void __launch_bounds__(kListThreads, 5)
     }
     for (int q = tid; q < n_dirs; q += kListThreads) s_dir[q] = dirs[q];
     for (int q = tid; q < C.total_steps; q += kListThreads) s_rl10[q] = C.rl10[q];
-    const int plane = B.wx * B.wy, texels = plane * B.wz, box = plane * (B.wz - 1);
+    const int plane = B.wx * B.wy, texels = plane * B.wz, records = plane * (B.wz - 1);
     for (int t = tid; t < texels; t += kListThreads) {
         const int row = t / B.wx, x = t - row * B.wx, z = row / B.wy, y = row - z * B.wy;
         const int ox = x - B.hx, oy = y - B.hy, oz = z - B.hz;
@@ -362,7 +388,7 @@ __global__ void __launch_bounds__(kListThreads, 5)
         for (int e = 0; e < per_block; ++e) {
             if (s_voxel[e] < 0) continue;
             const float3 at = s_centre[e];
-            stage_texel(s_boxes + e * box, t, z, B.wz, plane,
+            stage_texel(s_boxes + e * records, t, z, B.wz, plane,
                         tex3D<float2>(td_tex, at.x + (float)ox, at.y + (float)oy, at.z + (float)oz));
         }
     }
@@ -373,9 +399,10 @@ __global__ void __launch_bounds__(kListThreads, 5)
         const int e = q / n_dirs, d = q - e * n_dirs, c = d / 12;
         if (s_voxel[e] < 0) continue;
         const CccsVoxel V = s_geo[e];
-        const float4 own = s_boxes[e * box + B.hz * plane + B.hy * B.wx + B.hx];
-        s_x[e][d] = cccs_direction(C, B, c, s_rl10 + C.step_off[c], V.tilt(g, s_dir[d]), V.tc, b, sp_cm, td_tex,
-                                   s_boxes + e * box, B.wx, plane, cap, make_float2(own.x, own.z));
+        const RecordBox box{s_boxes + e * records, B.wx, plane, cap};
+        const float4 own = box.box[B.hz * plane + B.hy * B.wx + B.hx];
+        s_x[e][d] = cccs_direction(C, B, c, s_rl10 + C.step_off[c], V.tilt(g, s_dir[d]), V.tc, b, sp_cm, td_tex, box,
+                                   make_float2(own.x, own.z));
     }
     __syncthreads();
     const int e = tid / Tile::groups, group = tid % Tile::groups;
@@ -397,6 +424,155 @@ __global__ void __launch_bounds__(kListThreads, 5)
     }
 }
 
+// The same for long lists, where a box per voxel costs more than its samples.  A
+// block compacts its entries above the mask and works through them in runs: a
+// run is as many of the next entries as share a staged box that fits and holds
+// no more texels than a box for each would (neighbours along a row of a sorted
+// list do).  A run's pairs of direction and voxel are dealt to the threads,
+// voxels innermost, so that a warp's lanes march alike.  Boxes hold single
+// texels: half the shared memory, twice the blocks per SM.
+//
+// Measured (us; before = one thread per listed voxel, every sample from the
+// texture unit; in brackets a box per voxel), 10 x 10 cm fields: every voxel of 128^3
+// at 2.5 mm 1118 -> 907 (2540), of 95^3 at 2 mm 1307 -> 1340 (3263), of 96^3 at 1 mm 2621 ->
+// 2870 (14970); every other per axis 189 -> 198 (341), 215 -> 256 (430), 430 -> 520 (1980);
+// every fourth of 248^3 at 2.5 mm, 241 k, 92 -> 102 (137).  Where a box per voxel no
+// longer fits four to a block: 15 k of 96^3 at 1 mm 173 -> 182 (285).
+constexpr int kRunThreads = 256, kRunVoxels = 32, kRunEntries = 128;
+__global__ void __launch_bounds__(kRunThreads, 4)
+    cccs_runs_kernel(Grid g, Frame f, const __grid_constant__ CccsCones C, const __grid_constant__ CccsPlan B,
+                     int per_block, int most_texels, float sp_cm, float dose_scale, const float4 *__restrict__ dirs,
+                     cudaTextureObject_t td_tex, const float *__restrict__ electron, const int *__restrict__ voxels,
+                     int n, float *__restrict__ out) {
+    extern __shared__ float2 s_texels[];  // most_texels
+    __shared__ float4 s_dir[kMaxCones * 12];
+    __shared__ float s_rl10[kMaxConeSteps];
+    __shared__ float s_x[kMaxCones * 12 * kRunVoxels];
+    __shared__ CccsVoxel s_geo[kRunVoxels];
+    __shared__ int s_voxel[kRunEntries], s_entry[kRunEntries], s_count[kRunEntries / 32];
+    __shared__ int s_run[7];  // voxels, low corner, widths of the box
+    const int tid = threadIdx.x, lane = tid & 31, e0 = blockIdx.x * per_block, n_dirs = C.n_cones * 12;
+    auto index3 = [&](int v) {
+        const int row = v / g.nx, k = row / g.ny;
+        return make_int3(v - row * g.nx, row - k * g.ny, k);
+    };
+    int v = -1;
+    if (tid < kRunEntries) {
+        if (tid < per_block && e0 + tid < n) {
+            v = __ldg(voxels + e0 + tid);
+            if (v < 0 || (long long)v >= g.n()) v = -1;
+            if (v >= 0) {
+                // masked by the texel itself (read at its centre), which a fluence map may have scaled since the mask
+                const int3 q = index3(v);
+                if (tex3D<float2>(td_tex, q.x + 0.5f, q.y + 0.5f, q.z + 0.5f).x <= 0.01f) v = -1;
+            }
+            if (v < 0) out[e0 + tid] = 0.0f;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, v >= 0);
+        if (lane == 0) s_count[tid >> 5] = __popc(bal);
+    }
+    __syncthreads();
+    int left = 0, base = 0;
+#pragma unroll
+    for (int q = 0; q < kRunEntries / 32; ++q) {
+        base += q < (tid >> 5) ? s_count[q] : 0;
+        left += s_count[q];
+    }
+    if (left == 0) return;
+    if (tid < kRunEntries) {
+        const unsigned bal = __ballot_sync(0xffffffffu, v >= 0);
+        if (v >= 0) {
+            const int at = base + __popc(bal & ((1u << lane) - 1u));
+            s_voxel[at] = v;
+            s_entry[at] = e0 + tid;
+        }
+    }
+    for (int q = tid; q < n_dirs; q += kRunThreads) s_dir[q] = dirs[q];
+    for (int q = tid; q < C.total_steps; q += kRunThreads) s_rl10[q] = C.rl10[q];
+    __syncthreads();
+    const int single = (2 * B.hx + 2) * (2 * B.hy + 2) * (2 * B.hz + 2);  // texels of one voxel's box
+    for (int first = 0; left > 0;) {
+        if (tid < 32) {
+            const int3 q = index3(s_voxel[first + min(lane, left - 1)]);
+            int3 lo = q, hi = q;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int3 l = make_int3(__shfl_up_sync(0xffffffffu, lo.x, o), __shfl_up_sync(0xffffffffu, lo.y, o),
+                                         __shfl_up_sync(0xffffffffu, lo.z, o));
+                const int3 h = make_int3(__shfl_up_sync(0xffffffffu, hi.x, o), __shfl_up_sync(0xffffffffu, hi.y, o),
+                                         __shfl_up_sync(0xffffffffu, hi.z, o));
+                if (lane >= o) {
+                    lo = make_int3(min(lo.x, l.x), min(lo.y, l.y), min(lo.z, l.z));
+                    hi = make_int3(max(hi.x, h.x), max(hi.y, h.y), max(hi.z, h.z));
+                }
+            }
+            const int wx = hi.x - lo.x + 2 * B.hx + 2, wy = hi.y - lo.y + 2 * B.hy + 2, wz = hi.z - lo.z + 2 * B.hz + 2;
+            const bool fits = lane < left && max(wx, max(wy, wz)) <= 255 &&
+                              (long long)wx * wy * wz <= min(most_texels, single * (lane + 1));
+            const int last = 31 - __clz(__ballot_sync(0xffffffffu, fits));  // lane 0's box of its own always fits
+            if (lane == last) {
+                s_run[0] = last + 1;
+                s_run[1] = lo.x, s_run[2] = lo.y, s_run[3] = lo.z;
+                s_run[4] = wx, s_run[5] = wy, s_run[6] = wz;
+            }
+        }
+        __syncthreads();
+        const int m = s_run[0], wx = s_run[4], wy = s_run[5], wz = s_run[6], plane = wx * wy;
+        const int3 lo = make_int3(s_run[1], s_run[2], s_run[3]);
+        if (tid < m) {
+            const int3 q = index3(s_voxel[first + tid]);
+            s_geo[tid] = CccsVoxel(g, f, q.x, q.y, q.z);
+        }
+        {
+            int row = tid / wx, x = tid - row * wx, z = row / wy, y = row - z * wy;
+            const int drow = kRunThreads / wx, dx = kRunThreads - drow * wx, dz = drow / wy, dy = drow - dz * wy;
+            for (int t = tid; t < plane * wz; t += kRunThreads) {
+                s_texels[t] = tex3D<float2>(td_tex, (float)(lo.x - B.hx + x) + 0.5f, (float)(lo.y - B.hy + y) + 0.5f,
+                                            (float)(lo.z - B.hz + z) + 0.5f);
+                x += dx, y += dy, z += dz;
+                if (x >= wx) x -= wx, ++y;
+                if (y >= wy) y -= wy, ++z;
+            }
+        }
+        __syncthreads();
+        const TexelBox box{s_texels, wx, plane, (wz - 2) * plane + (wy - 2) * wx + wx - 2};
+        // voxels innermost, padded to a power of two: a thread keeps its voxel
+        const int bits = m > 1 ? 32 - __clz(m - 1) : 0, e = tid & ((1 << bits) - 1);
+        if (e < m) {
+            const int3 l = index3(s_voxel[first + e]);
+            const int3 at = make_int3(l.x - lo.x + B.hx, l.y - lo.y + B.hy, l.z - lo.z + B.hz);
+            const float3 b = make_float3((float)(at.x * 256) + kMagic, (float)(at.y * 256) + kMagic, (float)(at.z * 256) + kMagic);
+            const float2 own = s_texels[at.z * plane + at.y * wx + at.x];
+            const CccsVoxel V = s_geo[e];
+            int c = 0;
+            for (int d = tid >> bits; d < n_dirs; d += kRunThreads >> bits) {
+                while (d >= 12 * (c + 1)) ++c;
+                s_x[d * m + e] = cccs_direction(C, B, c, s_rl10 + C.step_off[c], V.tilt(g, s_dir[d]), V.tc, b, sp_cm, td_tex,
+                                                box, own);
+            }
+        }
+        __syncthreads();
+        if (tid < kRunVoxels * Tile::groups) {  // four neighbouring lanes add a voxel's groups, in their order
+            const int e = tid / Tile::groups, group = tid % Tile::groups;
+            float sum = 0.0f;
+            if (e < m)
+                for (int c = 0; c < C.n_cones; ++c) {
+                    float cone = 0.0f;
+                    for (int az = group; az < 12; az += Tile::groups)
+                        cone = fmaf(s_dir[c * 12 + az].w, s_x[(c * 12 + az) * m + e], cone);
+                    sum += cone;
+                }
+            float all = sum;
+#pragma unroll
+            for (int q = 1; q < Tile::groups; ++q) all += __shfl_sync(0xffffffffu, sum, (lane & ~(Tile::groups - 1)) + q);
+            if (group == 0 && e < m) out[s_entry[first + e]] = cccs_dose(all, __ldg(electron + s_voxel[first + e]), dose_scale);
+        }
+        first += m;
+        left -= m;
+        // s_run and s_geo are written again: the reads above lie before the barrier that follows the run's pairs
+    }
+}
+
 DC_BOUNDS_TAKE(take_bounds_cccs)
 
 namespace {
@@ -409,7 +585,7 @@ constexpr size_t kMostBytes = 104 * 1024;
 // function, and calls of several threads share it.
 template <class K>
 void allow_shared(K *kernel, size_t smem, int device, std::atomic<bool> (&done)[64]) {
-    if (smem <= 40 * 1024) return;  // the static arrays count too
+    if (smem <= 16 * 1024) return;  // the static arrays (up to 18 KB) count too
     if (device < 64 && done[device].load(std::memory_order_acquire)) return;
     DC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostBytes));
     if (device < 64) done[device].store(true, std::memory_order_release);
@@ -474,12 +650,30 @@ void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, cons
     KernelTimer kt(ctx, "cccs_points", s);
     CccsPlan B;
     cccs_plan(C, g, B);  // the tiles' split of the samples
+    const size_t texels = (size_t)(2 * B.hx + 2) * (2 * B.hy + 2) * (2 * B.hz + 2);  // of one voxel's box
+    const size_t box = texels / (2 * B.hz + 2) * (2 * B.hz + 1) * sizeof(float4);
+    // A box per voxel for short lists (100 k entries, 24 k where more than one voxel in 32 is listed: there
+    // neighbours share most of theirs), as long as at least three fit
+    const bool runs = 56 * 1024 / box < 3 || n >= 100000 || (n >= 24000 && 32LL * n >= g.n());
+    if (runs) {
+        const size_t one = texels * sizeof(float2);
+        const size_t smem = std::max(one, std::min<size_t>(30 * 1024, std::max<size_t>(20 * 1024, 8 * one)));
+        static std::atomic<bool> allowed[64] = {};
+        allow_shared(cccs_runs_kernel, smem, ctx.device, allowed);
+        // few entries per block keep a sparse list's many short runs apart; a dense one has long runs
+        const bool dense = 4LL * n >= g.n();
+        const int per_block = dense && n >= 500000 ? 128 : dense && n >= 200000 ? 64 : 16;
+        cccs_runs_kernel<<<(unsigned)((n + per_block - 1) / per_block), kRunThreads, smem, s>>>(
+            g, f, C, B, per_block, (int)(smem / sizeof(float2)), g.sx / 10.0f, dose_scale, w.dirs, w.td_tex, w.electron,
+            voxels, n, out);
+        check_launch("cccs_runs_kernel");
+        return;
+    }
     float reach = 0.0f;
     for (int c = 0; c < C.n_cones; ++c)
         if (B.n_near[c] > 0) reach = std::max(reach, C.rl10[C.step_off[c] + B.n_far[c]]);
     B.wx = 2 * B.hx + 2, B.wy = 2 * B.hy + 2, B.wz = 2 * B.hz + 2;
-    const size_t box = (size_t)B.wx * B.wy * (B.wz - 1) * sizeof(float4);
-    const int per_block = (int)std::min<size_t>(kListVoxels, std::max<size_t>(1, 56 * 1024 / box));
+    const int per_block = (int)std::min<size_t>(kListVoxels, 56 * 1024 / box);
     const size_t smem = box * per_block;
     static std::atomic<bool> allowed[64] = {};
     allow_shared(cccs_list_kernel, smem, ctx.device, allowed);

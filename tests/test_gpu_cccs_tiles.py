@@ -65,3 +65,39 @@ def _check(engine, oracle, vol, rho, grid, spacing, model, cp, rng):
     got = beam.probe(torch.as_tensor(pick, device="cuda")).cpu().numpy()
     assert np.array_equal(got[:-2], dose.ravel()[pick[:-2]]) and (got[-2:] == 0).all()
     beam.close()
+
+
+@pytest.mark.parametrize("shape,spacing,field,lists", [
+    ((40, 44, 52), (2.5, 2.5, 2.5), 40.0, ("all", "third", "shuffled")),   # a box per voxel, shared boxes
+    ((24, 30, 40), (1.0, 1.0, 1.0), 15.0, ("all", "third", "shuffled")),   # boxes too large for four per block
+    ((3, 70, 300), (2.0, 2.0, 2.0), 60.0, ("all", "third")),               # rows longer than a run, runs across rows
+    ((70, 60, 64), (3.0, 2.0, 2.5), 80.0, ("all",)),                       # more entries per block
+])
+def test_lists_equal_the_full_dose(shape, spacing, field, lists):
+    """A probe's dose is the full calculation's bit for bit, whichever way its list is worked through: every
+    voxel and every third in order, in any order with repeats, with entries outside the grid."""
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTControlPoint, IMRTPlan
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    rng = np.random.default_rng(sum(shape))
+    nz, ny, nx = shape
+    grid = types.SimpleNamespace(spacing=np.array(spacing), origin=np.array([-n * s / 2 for n, s in zip((nx, ny, nz), spacing)]))
+    x12 = np.where(np.abs(model.mlc_offsets) <= field / 2, field / 2, 0.0)
+    mlc = np.array(np.vstack((-x12, x12, model.mlc_offsets, model.mlc_widths)), dtype=np.single).T
+    cp = IMRTControlPoint(np.zeros(3, np.single), 100.0, mlc, 33.0, 0.0, 20.0, None, None)
+    beam = engine.PhotonBeam(grid, shape)
+    beam.set_density(torch.as_tensor(rng.uniform(0.2, 1.6, shape).astype(np.single), device="cuda"))
+    beam.terma(model, cp)
+    full = beam.dose().reshape(-1)
+    n = full.numel()
+    assert bool((full > 0).any()) and bool((full == 0).any())
+    for kind in lists:
+        pick = {"all": np.arange(n), "third": np.arange(1, n, 3), "shuffled": rng.integers(0, n, n)}[kind].astype(np.int32)
+        out = rng.integers(0, pick.size, 20)
+        pick[out[:10]], pick[out[10:]] = -1, n
+        v = torch.as_tensor(pick, device="cuda").long()
+        want = torch.where((v >= 0) & (v < n), full[v.clamp(0, n - 1)], torch.zeros((), device="cuda"))
+        for part in (pick.size, 5000):  # long and short
+            got = beam.probe(torch.as_tensor(pick[:part], device="cuda"))
+            assert torch.equal(got, want[:part])
+    beam.close()
