@@ -56,17 +56,21 @@ __global__ void __launch_bounds__(128) wet_march_kernel(Grid g, Frame f, cudaTex
 // take kBrick r - 1 voxels of steps, along the axis it crosses fastest, as
 // additions of c.  They are the plain march's additions in its order, so the
 // sum is the same bit for bit.  The map is built from the texture in every
-// call.
+// call, its radii only where enough bricks are uniform; otherwise the march
+// does not look at it.
 //
 // Measured on B200 (us, map + march, before -> after): 96^3 at 2 mm of water
-// with inserts 190 -> 20 + 67; 127 x 113 x 91 oblique 288 -> 20 + 228; 256 x
-// 256 x 160, noisy body in air 3735 -> 45 + 2360; the same filled with one
-// value 45 + 425, with noise in every voxel 42 + 3780 (the looks at the map
-// cost 1 %; every 4 samples instead of every 6 2 %, every 8 loses 3 % on the
-// body).  Bricks of 8 voxels gave 2750 on the body (fewer leaps near its
-// surface), of 2 voxels 2367 with a map of 210.  The photon depth's marched
-// voxels gain less than the map costs (their rays run through the noisy body)
-// and do not leap.
+// with inserts 190 -> 18 + 67; 127 x 113 x 91 oblique 288 -> 21 + 228; 256 x
+// 256 x 160, noisy body in air 3735 -> 50 + 2360; the same filled with one
+// value 51 + 414.  With noise in every voxel the map is a loss: 38 + 3711 there
+// (3710), 96^3 14 + 184 (186), 80^3 11 + 101 (104).  The looks at the map cost
+// 1 %; every 4 samples instead of every 6 2 %, every 8 loses 3 % on the body.
+// Bricks of 8 voxels gave 2750 on the body (fewer leaps near its surface), of 2
+// voxels 2367 with a map of 210.  Testing 256 bricks in a kernel of its own first
+// cost more than it saved (28 us instead of 17 where the map is made), so did
+// the eight-lane march as a second launch where nothing is uniform (its empty
+// blocks take 8 to 15 us).  The photon depth's marched voxels gain less than the
+// map costs (their rays run through the noisy body) and do not leap.
 constexpr int kBrick = 4;
 constexpr int kBrickRadius = 4;
 constexpr int kFetches = 6;  // samples fetched between two looks at the map
@@ -74,6 +78,8 @@ constexpr int kFetches = 6;  // samples fetched between two looks at the map
 struct Bricks {
     float *value = nullptr;           // NaN: not uniform
     unsigned char *radius = nullptr;  // 0: the brick or a neighbour differs
+    unsigned *uniform = nullptr;      // uniform bricks; with fewer than `least` of them nothing is leapt over
+    unsigned least = 0;
     int nx = 0, ny = 0, nz = 0;
 };
 
@@ -111,12 +117,11 @@ struct Leaps {
     }
 };
 
-// Value of each brick of the volume, NaN where its voxels differ (bit for
-// bit) or hold a number whose filtered value might not be exact.  A warp per
-// brick; reading at a texel's centre returns the stored value.
-__global__ void __launch_bounds__(128) brick_value_kernel(Grid g, Bricks B, cudaTextureObject_t density) {
-    const int b = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (b >= B.nx * B.ny * B.nz) return;
+// Value of a brick, NaN where its voxels differ (bit for bit) or hold a number
+// whose filtered value might not be exact.  By a warp; reading at a texel's
+// centre returns the stored value.
+__device__ __forceinline__ float brick_value(const Grid &g, const Bricks &B, cudaTextureObject_t density, int b) {
+    const int lane = threadIdx.x & 31;
     const int bz = b / (B.nx * B.ny), by = (b - bz * B.nx * B.ny) / B.nx, bx = b - (bz * B.ny + by) * B.nx;
     const int x0 = bx * kBrick, y0 = by * kBrick, z0 = bz * kBrick;
     const float c = tex3D<float>(density, x0 + 0.5f, y0 + 0.5f, z0 + 0.5f);
@@ -130,8 +135,24 @@ __global__ void __launch_bounds__(128) brick_value_kernel(Grid g, Bricks B, cuda
         same = same && __float_as_uint(tex3D<float>(density, i + 0.5f, j + 0.5f, k + 0.5f)) == __float_as_uint(c);
     }
     const bool plain = c == 0.0f || (fabsf(c) >= 1.0e-30f && fabsf(c) <= 1.0e30f);
-    same = __all_sync(0xffffffffu, same) && plain;
-    if (lane == 0 && DC_IN_BOUNDS(b, B.nx * B.ny * B.nz, 6)) B.value[b] = same ? c : NAN;
+    return __all_sync(0xffffffffu, same) && plain ? c : NAN;
+}
+
+// Values of all bricks, and the number of uniform ones (0 before).
+__global__ void __launch_bounds__(128) brick_value_kernel(Grid g, Bricks B, cudaTextureObject_t density) {
+    const int n = B.nx * B.ny * B.nz;
+    int uniform = 0;
+    for (int b = blockIdx.x * 4 + (threadIdx.x >> 5); b < n; b += gridDim.x * 4) {
+        const float c = brick_value(g, B, density, b);
+        uniform += c == c;
+        if ((threadIdx.x & 31) == 0 && DC_IN_BOUNDS(b, n, 6)) B.value[b] = c;
+    }
+    __shared__ int s_uniform;
+    if (threadIdx.x == 0) s_uniform = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && uniform > 0) atomicAdd(&s_uniform, uniform);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_uniform > 0) atomicAdd(B.uniform, (unsigned)s_uniform);
 }
 
 // Radius of each brick: the Chebyshev distance to the nearest brick of another
@@ -139,11 +160,12 @@ __global__ void __launch_bounds__(128) brick_value_kernel(Grid g, Bricks B, cuda
 // max(|dy|, that of the row dy away), then likewise along z; a block takes
 // kTile^3 bricks with their surroundings in shared memory.
 constexpr int kTile = 8, kSpan = kTile + 2 * kBrickRadius;
-__global__ void __launch_bounds__(256) brick_radius_kernel(Bricks B) {
+__global__ void __launch_bounds__(512) brick_radius_kernel(Bricks B) {
     __shared__ float val[kSpan][kSpan][kSpan];
     __shared__ unsigned char dx[kSpan][kSpan][kTile], dxy[kSpan][kTile][kTile];
+    if (*B.uniform < B.least) return;
     const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, z0 = blockIdx.z * kTile;
-    for (int e = threadIdx.x; e < kSpan * kSpan * kSpan; e += 256) {
+    for (int e = threadIdx.x; e < kSpan * kSpan * kSpan; e += 512) {
         const int lx = e % kSpan, ly = e / kSpan % kSpan, lz = e / (kSpan * kSpan);
         // outside the volume the nearest brick inside again, which adds no nearer difference
         const int x = min(max(x0 + lx - kBrickRadius, 0), B.nx - 1), y = min(max(y0 + ly - kBrickRadius, 0), B.ny - 1);
@@ -152,7 +174,7 @@ __global__ void __launch_bounds__(256) brick_radius_kernel(Bricks B) {
     }
     __syncthreads();
     constexpr int kFar = kBrickRadius + 1;
-    for (int e = threadIdx.x; e < kSpan * kSpan * kTile; e += 256) {
+    for (int e = threadIdx.x; e < kSpan * kSpan * kTile; e += 512) {
         const int lx = e % kTile, ly = e / kTile % kSpan, lz = e / (kTile * kSpan);
         const float c = val[lz][ly][lx + kBrickRadius];
         int d = kFar;
@@ -162,7 +184,7 @@ __global__ void __launch_bounds__(256) brick_radius_kernel(Bricks B) {
         dx[lz][ly][lx] = (unsigned char)d;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < kSpan * kTile * kTile; e += 256) {
+    for (int e = threadIdx.x; e < kSpan * kTile * kTile; e += 512) {
         const int lx = e % kTile, ly = e / kTile % kTile, lz = e / (kTile * kTile);
         const float c = val[lz][ly + kBrickRadius][lx + kBrickRadius];
         int d = kFar;
@@ -174,7 +196,7 @@ __global__ void __launch_bounds__(256) brick_radius_kernel(Bricks B) {
         dxy[lz][ly][lx] = (unsigned char)d;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < kTile * kTile * kTile; e += 256) {
+    for (int e = threadIdx.x; e < kTile * kTile * kTile; e += 512) {
         const int lx = e % kTile, ly = e / kTile % kTile, lz = e / (kTile * kTile);
         const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
         if (x >= B.nx || y >= B.ny || z >= B.nz) continue;
@@ -203,6 +225,7 @@ __global__ void __launch_bounds__(32 * kMarchZ) wet_march_leap_kernel(Grid g, Fr
     const float3 p = voxel_xyz(g, f, i, j, k);
     const float3 u = unit_to_source(f, p);
     const Leaps leaps(g, f, p, u);
+    const bool worth = *B.uniform >= B.least;
 
     float wet_sum = -0.05f;
     int t = 0;
@@ -220,7 +243,7 @@ __global__ void __launch_bounds__(32 * kMarchZ) wet_march_leap_kernel(Grid g, Fr
         inside = tex_inside(g, tc);
         if (!inside) break;
         float c;
-        const int n = leaps.at(B, tc, t, &c);
+        const int n = worth ? leaps.at(B, tc, t, &c) : 0;
         if (n > 0) {
             c = fmaxf(c, 0.0f);
 #pragma unroll 4
@@ -467,37 +490,42 @@ static Bricks brick_shape(const Grid &g) {
 
 size_t march_bytes(const Grid &g) {
     const Bricks B = brick_shape(g);
-    return (size_t)g.n() * sizeof(float) + (size_t)B.nx * B.ny * B.nz * (sizeof(float) + 1);
+    return (size_t)g.n() * sizeof(float) + (size_t)B.nx * B.ny * B.nz * (sizeof(float) + 1) + sizeof(unsigned);
 }
 
-// Whether the march leaps.  The map takes 14 to 45 us, so a march shorter than
-// some 90 us (4e7 samples, a voxel's mean path being half the volume's mean
-// extent) would win little and lose more where nothing is uniform: 80^3 at 2 mm
-// takes 92 us with eight lanes per ray; leaping 15 + 25 where all is uniform
-// and 15 + 104 where nothing is.
-static bool march_leaps(const Grid &g) {
-    const double mean = (g.nx * (double)g.sx + g.ny * (double)g.sy + g.nz * (double)g.sz) / 6.0;  // mm to the boundary
-    return (double)g.n() * mean > 4.0e7;
+// Samples of a plain march: a voxel's mean path is half the volume's mean extent.
+static double march_samples(const Grid &g) {
+    return (double)g.n() * (g.nx * (double)g.sx + g.ny * (double)g.sy + g.nz * (double)g.sz) / 6.0;
 }
 
 static Bricks launch_bricks(DeviceContext &ctx, const Grid &g, cudaTextureObject_t density, float *wet, cudaStream_t s) {
     Bricks B = brick_shape(g);
     const long long n = (long long)B.nx * B.ny * B.nz;
     B.value = wet + g.n();
-    B.radius = reinterpret_cast<unsigned char *>(B.value + n);
+    B.uniform = reinterpret_cast<unsigned *>(B.value + n);
+    B.radius = reinterpret_cast<unsigned char *>(B.uniform + 1);
+    // the rest of the map and the looks at it pay off from some 6 % of uniform bricks on, in short marches 20 %
+    B.least = (unsigned)((double)n * (0.06 + 0.15 * 4.0e7 / march_samples(g)));
     KernelTimer kt(ctx, "march_bricks", s);
-    brick_value_kernel<<<(unsigned)((n + 3) / 4), 128, 0, s>>>(g, B, density);
+    int sms = 0;
+    DC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+    DC_CUDA(cudaMemsetAsync(B.uniform, 0, sizeof(unsigned), s));
+    brick_value_kernel<<<(unsigned)std::min((n + 3) / 4, 32LL * sms), 128, 0, s>>>(g, B, density);
     check_launch("brick_value_kernel");
     const dim3 tiles((unsigned)((B.nx + kTile - 1) / kTile), (unsigned)((B.ny + kTile - 1) / kTile),
                      (unsigned)((B.nz + kTile - 1) / kTile));
-    brick_radius_kernel<<<tiles, 256, 0, s>>>(B);
+    brick_radius_kernel<<<tiles, 512, 0, s>>>(B);
     check_launch("brick_radius_kernel");
     return B;
 }
 
+// Whether the march may leap.  The map takes 11 to 20 us, so a march shorter than
+// some 90 us (4e7 samples) would win little: 80^3 at 2 mm takes 91 us with eight
+// lanes per ray; leaping 16 + 21 where all is uniform, 15 + 65 for a body in
+// uniform air and 11 + 102 where nothing is.
 void launch_wet_march(DeviceContext &ctx, const Grid &g, const Frame &f, cudaTextureObject_t density,
                       float *wet, cudaStream_t s) {
-    if (march_leaps(g)) {
+    if (march_samples(g) > 4.0e7) {
         const Bricks B = launch_bricks(ctx, g, density, wet, s);
         KernelTimer kt(ctx, "wet_march", s);
         const dim3 grid((unsigned)((g.nx + kMarchX - 1) / kMarchX), (unsigned)((g.ny + kMarchY - 1) / kMarchY),

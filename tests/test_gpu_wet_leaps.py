@@ -42,3 +42,26 @@ def test_leaps_equal_the_sampled_march(shape, spacing, gantry, couch):
     # here: a few voxels beside an edge stand on such a step and move with the last place
     far = np.abs(wet[0] - wet[1])[deep] > 512 * 2.0 ** -23 * wet[1][deep]
     assert far.mean() < 1e-5
+
+
+@pytest.mark.parametrize("part", [0.0, 0.03, 0.3])
+def test_volumes_mostly_of_noise(part):
+    """Below some 6 to 20 % of uniform bricks nothing is leapt over; above, the uniform part is.  Either way the
+    sums are those of the samples: against the volume whose uniform part is moved by one unit in the last
+    place in a checkerboard, as above."""
+    import torch
+
+    from dosecuda_b200 import engine
+    nz, ny, nx = shape = (90, 97, 101)
+    rho = np.random.default_rng(4).uniform(0.7, 1.3, shape).astype(np.float32)
+    rho[: int(nz * part)] = 1.013
+    odd = np.indices(shape).sum(0) % 2 == 1
+    moved = np.where(odd & (rho == np.float32(1.013)), np.nextafter(rho, np.float32(2)), rho).astype(np.float32)
+    grid = types.SimpleNamespace(spacing=np.array([2.0] * 3), origin=np.array([-n * 1.0 for n in (nx, ny, nz)]))
+    beam = types.SimpleNamespace(iso=np.zeros(3, np.float32), gantry_angle=20.0, couch_angle=70.0)
+    model = types.SimpleNamespace(VSADX=2000.0, VSADY=1800.0)
+    wet = [engine.proton_wet(torch.as_tensor(v, device="cuda"), grid, beam, model).cpu().numpy() for v in (rho, moved)]
+    deep = wet[1] > 1.1
+    assert deep.mean() > 0.5
+    far = np.abs(wet[0] - wet[1])[deep] > 512 * 2.0 ** -23 * wet[1][deep]
+    assert far.mean() < 1e-5
