@@ -491,14 +491,17 @@ class ProtonBatch:
         keep the fastest; results are cached in ``cache_path`` (JSON)."""
         import json
         import os
-        key = "%s|%d plans|%d beams|%d spots|%s" % (
-            torch.cuda.get_device_name(self.device), self.n_plans, self.n_beams, self.n_spots,
+        # names what a variant number stands for (dc_pencil.cu's kBatchWarps): numbers
+        # that an older build of the kernel cached meant other shapes
+        layers = sum(len(np.unique(sp[:, 3].astype(np.int64))) for sp in self.beam_spots)
+        key = "warps per block 4,2,1,7|%s|%d plans|%d beams|%d layers|%d spots|%s" % (
+            torch.cuda.get_device_name(self.device), self.n_plans, self.n_beams, layers, self.n_spots,
             ";".join("x".join(str(d) for d in r.shape) for r in self.rlsp))
         cache = {}
         if cache_path and os.path.exists(cache_path):
             with open(cache_path) as f:
                 cache = json.load(f)
-        if key in cache:
+        if key in cache and 0 <= int(cache[key]["variant"]) < self.n_variants:
             self.variant = int(cache[key]["variant"])
             return self.variant
         times = []

@@ -119,6 +119,25 @@ def test_tile_variants_agree_and_autotune(batch, tmp_path):
     assert b.autotune(str(cache)) == v  # served from the cache
 
 
+def test_autotune_ignores_other_kernels_and_bad_numbers(batch, tmp_path):
+    """Cached numbers written for other kernel variants (a key that did not name them), or out of range, are
+    not used: the shapes are timed again."""
+    import json
+    torch, engine, model, b, plans = batch
+    cache = tmp_path / "tune.json"
+    old = "%s|%d plans|%d beams|%d spots|%s" % (
+        torch.cuda.get_device_name(b.device), b.n_plans, b.n_beams, b.n_spots,
+        ";".join("x".join(str(d) for d in r.shape) for r in b.rlsp))
+    cache.write_text(json.dumps({old: {"variant": 2, "ms": []}}))
+    b.tune_ms = None
+    b.autotune(str(cache))
+    assert b.tune_ms is not None
+    new, = set(json.loads(cache.read_text())) - {old}
+    cache.write_text(json.dumps({new: {"variant": 99, "ms": []}}))
+    b.tune_ms = None
+    assert 0 <= b.autotune(str(cache)) < b.n_variants and b.tune_ms is not None
+
+
 def test_weights_and_cuda_graph_replay(batch):
     torch, engine, model, b, plans = batch
     mu = b.mu0.clone()
