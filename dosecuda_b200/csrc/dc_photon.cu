@@ -120,7 +120,7 @@ __device__ __forceinline__ float head_transmission(const PhotonParams &P, float3
             cached_xl = xl;
             cached_xr = xr;
         }
-        if (cached_ex == 0.0f) continue;  // beside the leaves: adds exactly 0
+        if (searched && cached_ex == 0.0f) continue;  // beside the leaves: adds exactly 0 (the y edges are finite)
         const float erf_b = (yb == cached_y) ? cached_erf_y : erff(a1);
         const float erf_t = erff(a2);
         cached_y = yt;

@@ -54,3 +54,22 @@ def test_terma_equals_that_of_unmergeable_pairs(kind):
         terma.append(beam.terma(model, cp, out=True).cpu().numpy())
     assert terma[0].max() > 0.1
     assert np.abs(terma[0] - terma[1]).max() <= 5e-6 * terma[0].max()
+
+
+def test_leaf_edge_that_is_not_a_number():
+    """A leaf pair at a y position of NaN makes TERMA NaN everywhere, also far beside the opening (here up to
+    0.8 m), where the pair's x factor is exactly 0."""
+    import torch
+
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTControlPoint, IMRTPlan
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    x1, x2, off, wid = _leaves("square", model).T.copy()
+    off[len(off) // 2] = np.nan
+    shape = (3, 4, 200)
+    grid = types.SimpleNamespace(spacing=np.array([8.0, 4.0, 4.0]), origin=np.array([-800.0, -8.0, -6.0]))
+    mlc = np.array(np.vstack((x1, x2, off, wid)), dtype=np.single).T
+    cp = IMRTControlPoint(np.zeros(3, np.single), 100.0, mlc, 0.0, 0.0, 0.0, None, None)
+    beam = engine.PhotonBeam(grid, shape)
+    beam.set_density(torch.ones(shape, device="cuda"))
+    assert bool(beam.terma(model, cp, out=True).isnan().all())
