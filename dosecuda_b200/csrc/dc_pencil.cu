@@ -512,7 +512,11 @@ __global__ void __launch_bounds__(32 * kWarps, 7)
 }
 
 // Voxel-list kernel: a warp takes 128 consecutive list entries, 32 per step
-// (a sorted list keeps them close together).
+// (a sorted list keeps them close together).  A voxel's distances and the split
+// of its layers are its own; the cut-offs are the warp's.  In another list the
+// same voxel may lose or gain terms beyond 6 sigma_ht (1.5e-8 of the halo's peak
+// each) and primaries below 2^-26 of their halo term, and add its spots in
+// another order.
 template <bool kAdj>
 __global__ void __launch_bounds__(32 * kWarps, 6)
     pencil_list_kernel(Grid g, Frame f, ProtonTables t, const float *__restrict__ wet_s, PbExtra x, int split) {
@@ -681,7 +685,7 @@ void list_launch(DeviceContext &ctx, const char *name, const Grid &g, const Fram
                  const float *wet_s, const PbExtra &x, cudaStream_t s) {
     if (x.n_list <= 0) return;
     const long long tiles = ((long long)x.n_list + kWarpVox - 1) / kWarpVox;
-    const int split = layer_split(ctx, 0, t.n_layers);  // the same for every list, as a voxel's dose is
+    const int split = layer_split(ctx, 0, t.n_layers);  // the same for every list, so that the layers' parts are
     const long long per = kWarps / split;
     constexpr size_t smem = kWarps * sizeof(WarpMem<kAdj>);
     KernelTimer kt(ctx, name, s);
