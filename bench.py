@@ -35,13 +35,13 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
-# DRAM bytes (read + write) per launch from one ncu --set full capture of each
+# DRAM bytes (read + write) per launch from one ncu capture of each
 # dominant kernel on these workloads, with the summary that records the
 # capture (its command and figures).  A kernel change makes its entry stale
 # until it is captured again.
 NCU_TRAFFIC = {
-    "cccs": (12782592, "profiles/cccs_photon_small.md"),
-    "pencil_beam": (4148480 + 50432, "profiles/pencil_beam_proton_small.md"),
+    "cccs": (12750000, "profiles/cccs_photon_small.md"),
+    "pencil_beam": (4150000, "profiles/pencil_beam_proton_small.md"),
     "conv_dec0": (67162880 + 26884352, "profiles/conv_gather_dec0_surrogate_128.md"),
 }
 SM_COUNT = 148

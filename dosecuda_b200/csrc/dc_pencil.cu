@@ -18,6 +18,9 @@
 //    for every voxel of the tile the primary term is below a quarter ulp of
 //    the halo term of the same pair and is not evaluated (the primary falls
 //    off within ~7 sigma_t, the halo's reach is 6 sigma_ht, about twice that).
+//    It counts where sigma_t is narrow: 65 % of the evaluated pairs of 256 x 256 x
+//    160, 32 % of 96^3, but 5 % of the listed voxels' and 0.3 % of the oblique
+//    beam's with its range shifter below.
 //  * r^2 = U^2 + W^2 with U, W the components of the voxel along two unit
 //    vectors normal to the spot's axis, taken relative to the tile's centre.
 //    Along the thread's four voxels r^2 is a parabola: 15 operations give the
@@ -27,10 +30,10 @@
 //
 // Measured on B200 (ms; before = the 16 x 8 x 4 tile per block of 256 threads
 // with its per-layer barriers): 96^3 beam of 2034 spots 0.95 -> 0.41; oblique
-// 127 x 113 x 91 with range shifter, 2831 spots 1.08 -> 0.62; 256 x 256 x 160,
+// 127 x 113 x 91 with range shifter, 2831 spots 1.08 -> 0.63; 256 x 256 x 160,
 // 2655 spots 2.32 -> 1.27; six beams of 160 x 160 x 96 in one batch 5.90 ->
-// 2.83; dose / adjoint at 105 k listed voxels, 6025 spots 0.48 -> 0.29 / 1.63
-// -> 0.29.  Of the batch's cycles the exponentials take 62 %.  Fewer or more
+// 2.86; dose / adjoint at 50 k listed voxels, 6025 spots 0.48 -> 0.30 / 1.63
+// -> 0.31.  Of the batch's cycles the exponentials take 62 %.  Fewer or more
 // registers (24 to 40 warps per SM) changed nothing above 1 %; evaluating a
 // quarter of the exponentials as polynomials on the FP32 pipe cost 5 %, tiles
 // of 8 x 4 x 8 voxels 4 to 15 %.

@@ -472,7 +472,9 @@ int dc_photon_beam_probe_select(dc_photon_beam *beam, int *n_out, void *stream);
 /* The selected list: device pointer and count, and optionally a host copy
  * of the first `cap` indices. */
 int dc_photon_beam_probe_list(const dc_photon_beam *beam, const int **voxels_dev, int *n, int *voxels_host, int cap);
-/* CCCS dose at n listed voxels (voxels_dev NULL: the selected list). */
+/* CCCS dose at n listed voxels (voxels_dev NULL: the selected list): 0 where
+ * the TERMA in the beam is at most 0.01 and outside the grid, elsewhere the
+ * full dose bit for bit. */
 int dc_photon_beam_probe(dc_photon_beam *beam, const int *voxels_dev, int n, float *dose_out_dev, void *stream);
 
 /* No counterpart in the reference (its TERMA has no fluence input,
