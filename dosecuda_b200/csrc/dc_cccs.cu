@@ -44,7 +44,6 @@
 // texels; one voxel more of margin, 5355, made it 2.65, and a 2 cm field 0.28
 // instead of 0.24).
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <type_traits>
 
@@ -580,15 +579,13 @@ namespace {
 // Most bytes of a staged box: two blocks per SM.
 constexpr size_t kMostBytes = 104 * 1024;
 
-// Opts the kernel in to kMostBytes of dynamic shared memory, once per device
-// and to the same limit whatever the launch needs: the limit belongs to the
+// Opts a kernel with `fixed` bytes of static shared memory in to kMostBytes of
+// dynamic, where the launch needs it.  Always the same limit: it belongs to the
 // function, and calls of several threads share it.
 template <class K>
-void allow_shared(K *kernel, size_t smem, int device, std::atomic<bool> (&done)[64]) {
-    if (smem <= 16 * 1024) return;  // the static arrays (up to 18 KB) count too
-    if (device < 64 && done[device].load(std::memory_order_acquire)) return;
-    DC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostBytes));
-    if (device < 64) done[device].store(true, std::memory_order_release);
+void allow_shared(K *kernel, size_t fixed, size_t smem) {
+    if (smem + fixed > 48 * 1024)
+        DC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostBytes));
 }
 
 // Fills B for a tile and returns the staged box's bytes.  Where no near sample
@@ -635,8 +632,7 @@ void enqueue_cccs(DeviceContext &ctx, const Grid &g, const Frame &f, const CccsC
     KernelTimer kt(ctx, "cccs", s);
     CccsPlan B;
     const size_t smem = cccs_plan(C, g, B);
-    static std::atomic<bool> allowed[64] = {};
-    allow_shared(cccs_kernel, smem, ctx.device, allowed);
+    allow_shared(cccs_kernel, 8 * 1024, smem);
     const dim3 grid((unsigned)((g.nx + Tile::x - 1) / Tile::x), (unsigned)((g.ny + Tile::y - 1) / Tile::y),
                     (unsigned)((g.nz + Tile::z - 1) / Tile::z));
     cccs_kernel<<<grid, kThreads, smem, s>>>(g, f, C, B, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex, w.electron, w.mask,
@@ -658,8 +654,7 @@ void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, cons
     if (runs) {
         const size_t one = texels * sizeof(float2);
         const size_t smem = std::max(one, std::min<size_t>(30 * 1024, std::max<size_t>(20 * 1024, 8 * one)));
-        static std::atomic<bool> allowed[64] = {};
-        allow_shared(cccs_runs_kernel, smem, ctx.device, allowed);
+        allow_shared(cccs_runs_kernel, 20 * 1024, smem);
         // few entries per block keep a sparse list's many short runs apart; a dense one has long runs
         const bool dense = 4LL * n >= g.n();
         const int per_block = dense && n >= 500000 ? 128 : dense && n >= 200000 ? 64 : 16;
@@ -675,8 +670,7 @@ void enqueue_cccs_points(DeviceContext &ctx, const Grid &g, const Frame &f, cons
     B.wx = 2 * B.hx + 2, B.wy = 2 * B.hy + 2, B.wz = 2 * B.hz + 2;
     const int per_block = (int)std::min<size_t>(kListVoxels, 56 * 1024 / box);
     const size_t smem = box * per_block;
-    static std::atomic<bool> allowed[64] = {};
-    allow_shared(cccs_list_kernel, smem, ctx.device, allowed);
+    allow_shared(cccs_list_kernel, 8 * 1024, smem);
     cccs_list_kernel<<<(unsigned)((n + per_block - 1) / per_block), kListThreads, smem, s>>>(
         g, f, C, B, per_block, reach * 1.0001f, g.sx / 10.0f, dose_scale, w.dirs, w.td_tex, w.electron, voxels, n,
         out);
