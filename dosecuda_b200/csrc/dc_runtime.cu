@@ -277,38 +277,51 @@ void DeviceContext::release_all() {
 }
 
 cudaEvent_t DeviceContext::take_event() {
-    if (!event_pool.empty()) {
-        cudaEvent_t e = event_pool.back();
-        event_pool.pop_back();
-        return e;
+    {
+        std::lock_guard<std::mutex> lk(prof_mu);
+        if (!event_pool.empty()) {
+            cudaEvent_t e = event_pool.back();
+            event_pool.pop_back();
+            return e;
+        }
     }
     cudaEvent_t e;
     DC_CUDA(cudaEventCreate(&e));
     return e;
 }
 
-void DeviceContext::prof_begin(const char *name, cudaStream_t s, cudaEvent_t *a, cudaEvent_t *b) {
+void DeviceContext::prof_begin(cudaStream_t s, cudaEvent_t *a, cudaEvent_t *b) {
     *a = take_event();
     *b = take_event();
-    pending.push_back({name, *a, *b});
     DC_CUDA(cudaEventRecord(*a, s));
 }
 
-void DeviceContext::prof_end(cudaEvent_t b, cudaStream_t s) { cudaEventRecord(b, s); }
+// Listed once both events are recorded, so that a collection on another thread
+// never waits for one that is not.
+void DeviceContext::prof_end(const char *name, cudaEvent_t a, cudaEvent_t b, cudaStream_t s) {
+    cudaEventRecord(b, s);
+    std::lock_guard<std::mutex> lk(prof_mu);
+    pending.push_back({name, a, b});
+}
 
 void DeviceContext::prof_collect() {
     DC_CUDA(cudaSetDevice(device));
-    for (auto &p : pending) {
+    std::vector<Pending> done;
+    {
+        std::lock_guard<std::mutex> lk(prof_mu);
+        done.swap(pending);
+    }
+    for (auto &p : done) {
         DC_CUDA(cudaEventSynchronize(p.b));
         float ms = 0.f;
         DC_CUDA(cudaEventElapsedTime(&ms, p.a, p.b));
         auto &e = profile[p.name];
         e.launches += 1;
         e.total_ms += ms;
+        std::lock_guard<std::mutex> lk(prof_mu);
         event_pool.push_back(p.a);
         event_pool.push_back(p.b);
     }
-    pending.clear();
 }
 
 // ---------------------------------------------------------------------------

@@ -156,8 +156,10 @@ class DeviceContext {
     void end_call(cudaStream_t s);
     static bool capturing(cudaStream_t s);
 
-    // Profiler.
+    // Profiler.  Kernels are timed by calls that hold `mu` and by calls that do
+    // not (a photon beam's), so pending and event_pool have a lock of their own.
     bool profiling = false;
+    std::mutex prof_mu;
     struct Pending {
         std::string name;
         cudaEvent_t a, b;
@@ -165,9 +167,9 @@ class DeviceContext {
     std::vector<Pending> pending;
     std::vector<cudaEvent_t> event_pool;
     std::map<std::string, ProfileEntry> profile;
-    void prof_begin(const char *name, cudaStream_t s, cudaEvent_t *a, cudaEvent_t *b);
-    void prof_end(cudaEvent_t b, cudaStream_t s);
-    void prof_collect();  // synchronises the device
+    void prof_begin(cudaStream_t s, cudaEvent_t *a, cudaEvent_t *b);
+    void prof_end(const char *name, cudaEvent_t a, cudaEvent_t b, cudaStream_t s);
+    void prof_collect();  // waits for the timed kernels; callers hold mu
     void release_all();
 
    private:
@@ -185,14 +187,15 @@ void release_context(int device);
 // profiler is enabled, CUDA events around the kernel.
 struct KernelTimer {
     DeviceContext &ctx;
+    const char *name;
     cudaStream_t s;
     cudaEvent_t a = nullptr, b = nullptr;
-    KernelTimer(DeviceContext &c, const char *name, cudaStream_t st) : ctx(c), s(st) {
+    KernelTimer(DeviceContext &c, const char *n, cudaStream_t st) : ctx(c), name(n), s(st) {
         nvtxRangePushA(name);
-        if (ctx.profiling && !DeviceContext::capturing(s)) ctx.prof_begin(name, s, &a, &b);
+        if (ctx.profiling && !DeviceContext::capturing(s)) ctx.prof_begin(s, &a, &b);
     }
     ~KernelTimer() {
-        if (b) ctx.prof_end(b, s);
+        if (b) ctx.prof_end(name, a, b, s);
         nvtxRangePop();
     }
 };

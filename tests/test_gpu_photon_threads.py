@@ -99,3 +99,44 @@ def test_termas_of_two_beams_on_two_streams():
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_kernels_timed_from_several_threads():
+    """With the kernel profiler on, photon beams on several threads time their kernels while another thread reads
+    the profile: every launch is counted once."""
+    import torch
+
+    from dosecuda_b200 import engine
+    from dosecuda_b200.plan_imrt import IMRTPlan
+    model = IMRTPlan("VarianTrueBeamHF").beam_models[0]
+    beams = [_beam(engine, model, (8, 12, 16), 3.0, 25.0) for _ in range(3)]
+    outs = [torch.empty((8, 12, 16), device="cuda") for _ in beams]
+    streams = [torch.cuda.Stream() for _ in beams]
+    for (b, cp), o in zip(beams, outs):
+        b.terma(model, cp)
+        b.dose(out=o)
+    torch.cuda.synchronize()
+    failed, n = [], 200
+
+    def work(q):
+        try:
+            for _ in range(n):
+                beams[q][0].dose(out=outs[q], stream=streams[q])
+        except Exception as e:
+            failed.append(e)
+
+    engine.profile(0, enable=True, reset=True)
+    try:
+        threads = [threading.Thread(target=work, args=(q,)) for q in range(len(beams))]
+        for t in threads:
+            t.start()
+        for _ in range(20):
+            engine.profile(0)
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        counted = engine.profile(0)["cccs"][0]
+    finally:
+        engine.profile(0, enable=False)
+    assert not failed, failed[0]
+    assert counted == n * len(beams)
